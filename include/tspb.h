@@ -297,10 +297,11 @@ int tspb_nn_init_jobs_smem(const tspb_nn_job* jobs, int32_t num_jobs, int32_t ma
  * (cpu_three_opt_best_move / cpu_three_opt_refine,
  * benchmark_scripts/experiments-and-examples/experiment-comparing-3opt-and-2opt/gpu_three_opt.py:143-277;
  * the GPU strategy LocalSearchGPUThreeOpt(mode="batch"/"naive") of the same file). Distances
- * from `dist` (n x dist_stride) or rebuilt from EUC_2D `coords`. One CTA per tour, `threads`
- * 128, 256 or 512; n <= 4096 (one pass is n^3/6 triples). For n above 220 each CTA needs n*n int32 of `workspace`
- * (tspb_three_opt_workspace_bytes); fewer CTAs are launched when the workspace holds fewer
- * tours (TSPB_ERR_WORKSPACE when it holds none). stats (optional): [tours][3] passes, moves,
+ * from `dist` (n x dist_stride) or rebuilt from EUC_2D `coords`. One CTA per tour, or a
+ * cluster of up to eight where the batch leaves SMs idle; `threads` is 128, 256 or 512 (checked;
+ * the CTA size is the library's). n <= 4096 (one pass is n^3/6 triples). For n above 220 each
+ * tour in flight needs n*n int32 of `workspace` (tspb_three_opt_workspace_bytes); fewer tours
+ * run at once when the workspace holds fewer (TSPB_ERR_WORKSPACE when it holds none). stats (optional): [tours][3] passes, moves,
  * (triple, case) candidates evaluated.
  */
 int tspb_three_opt(int32_t* tours, int32_t num_tours, int32_t n, const int32_t* dist, int64_t dist_stride,
