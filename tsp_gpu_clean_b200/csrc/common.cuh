@@ -43,6 +43,41 @@ struct DistSrc {
   }
 };
 
+// *p where `ok`, else 0, as one predicated load (L2 only, like the matrix reads above). A
+// conditional load written as a branch ends up beside the use of its value, so several of
+// them run one L2 round trip after another; the predicated form keeps them all in flight.
+__device__ __forceinline__ int load_cg_if(bool ok, const int32_t* p) {
+  int v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.cg.s32 %0, [%1];\n\t}"
+      : "=r"(v)
+      : "l"(p), "r"((int)ok));
+  return v;
+}
+
+// The same through the read-only path (L1), for the k-NN tables.
+__device__ __forceinline__ uint32_t load_nc_if(bool ok, const void* p) {
+  uint32_t v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}"
+      : "=r"(v)
+      : "l"(p), "r"((int)ok));
+  return v;
+}
+
+// d(a, b[u]) for the entries with ok[u] (0 elsewhere), all loads in flight together.
+template <int U>
+__device__ __forceinline__ void gather_if(const DistSrc& ds, int a, const int (&b)[U], const bool (&ok)[U], int (&d)[U]) {
+  if (ds.dist != nullptr) {
+    const int32_t* row = ds.dist + (long long)a * ds.stride;
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u] = load_cg_if(ok[u], row + b[u]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u] = ok[u] ? ds(a, b[u]) : 0;
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_min(T v) {
 #pragma unroll
@@ -53,6 +88,20 @@ __device__ __forceinline__ T warp_min(T v) {
   return v;
 }
 
+// 32- and 64-bit keys by the warp's hardware reduction (two of them for 64 bits: the high
+// words, then the low words of the lanes that hold that minimum) instead of five rounds of
+// shuffles.
+template <>
+__device__ __forceinline__ unsigned warp_min<unsigned>(unsigned v) {
+  return __reduce_min_sync(FULL, v);
+}
+template <>
+__device__ __forceinline__ unsigned long long warp_min<unsigned long long>(unsigned long long v) {
+  const unsigned hi = __reduce_min_sync(FULL, (unsigned)(v >> 32));
+  const unsigned lo = __reduce_min_sync(FULL, (unsigned)(v >> 32) == hi ? (unsigned)v : ~0u);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
@@ -60,7 +109,8 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// Block-wide min; `scratch` holds >= 32 T. Every thread gets the result.
+// Block-wide min of a block of whole warps; `scratch` holds >= 32 T. Every thread gets the
+// result.
 template <typename T>
 __device__ __forceinline__ T block_min(T v, T* scratch) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -68,9 +118,7 @@ __device__ __forceinline__ T block_min(T v, T* scratch) {
   __syncthreads();
   if (lane == 0) scratch[wid] = v;
   __syncthreads();
-  T r = scratch[0];
-  for (int w = 1; w < nw; ++w) r = scratch[w] < r ? scratch[w] : r;
-  return r;
+  return warp_min(scratch[lane < nw ? lane : 0]);
 }
 
 template <typename T>

@@ -20,6 +20,7 @@ struct TwoOptArgs {
   size_t ws_tour_bytes;
   size_t ws_keys_off;  // offset of the multi_move key buffer inside a tour's slice
   int arrays_in_smem;
+  int keys_in_smem;  // multi_move: slots of the key list held in shared memory
   const int32_t* rev_off;  // cached kernel: CSR offsets of the reverse k-NN index (n + 1)
   const int32_t* rev_idx;  // cached kernel: flat entries a * k + r grouped by candidate node
   const uint32_t* cand_packed;  // scan kernel: c | d(a, c) << 16 per entry (optional)
@@ -46,9 +47,11 @@ constexpr long long BUDGET_CYCLES = 1LL << 36;
 long long watchdog_cycles();
 
 int smem_optin();
+int device_attr(cudaDeviceAttr attr);
 size_t align256(size_t v);
 int launch_two_opt_cached(const TwoOptArgs& a, int mode, int threads, cudaStream_t st);
 size_t two_opt_cached_tour_bytes(int n, int mode);
+int launch_two_opt_multi(const TwoOptArgs& a, int threads, size_t smem, cudaStream_t st);
 int launch_two_opt_scan(const TwoOptArgs& a, int mode, int threads, cudaStream_t st);
 size_t two_opt_scan_tour_bytes(int n, int mode);
 int carveout_for(int ctas_per_sm, size_t smem_per_cta);

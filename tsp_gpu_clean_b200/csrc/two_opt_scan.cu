@@ -52,14 +52,14 @@ static bool scan_counts(const TwoOptArgs& a, int mode) { return mode == TSPB_MOD
 // tables. The default lets the driver take the largest split, which leaves too little L1.
 // An attribute of the current device (queried on every call: a process may drive GPUs of
 // different models, and the query is cheap next to a launch).
-static int current_device_attr(cudaDeviceAttr attr) {
+int device_attr(cudaDeviceAttr attr) {
   int dev = 0, v = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, attr, dev) != cudaSuccess) return 0;
   return v;
 }
 
 int carveout_for(int ctas_per_sm, size_t smem_per_cta) {
-  const int smem_sm = current_device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
+  const int smem_sm = device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
   if (smem_sm <= 0 || ctas_per_sm <= 0) return -1;
   const long long need = (long long)ctas_per_sm * (long long)(smem_per_cta + sizeof(ScanSmem) + 1024);
   int pct = (int)((need * 100 + smem_sm - 1) / smem_sm);
@@ -67,7 +67,7 @@ int carveout_for(int ctas_per_sm, size_t smem_per_cta) {
 }
 
 static int carveout_percent(int num_tours, size_t smem_per_cta, int max_ctas_per_sm) {
-  const int sms = current_device_attr(cudaDevAttrMultiProcessorCount);
+  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
   if (sms <= 0) return -1;
   int per_sm = (num_tours + sms - 1) / sms;
   if (per_sm > max_ctas_per_sm) per_sm = max_ctas_per_sm;
