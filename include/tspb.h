@@ -84,7 +84,9 @@ size_t tspb_two_opt_workspace_bytes(int32_t num_tours, int32_t n, int32_t k, int
  * distance in one word; given together with `rev_off`/`rev_idx`, first mode restarts
  * incrementally: after a move with window [bi, bj] a pass evaluates only the entries of
  * rows before bi whose candidate lies in the window, then scans from row bi (the other
- * entries before bi cannot have changed). Results and stats[0..2] are the same either way.
+ * entries before bi cannot have changed); best mode, where a full rescan is long enough,
+ * keeps every row's minimum and evaluates only what the last move can have changed. Results
+ * and stats[0..2] are the same either way.
  * Distances come from `dist` when non-NULL, else are rebuilt from `coords` in FP64
  * with TSPLIB EUC_2D rounding. `max_iterations` bounds the passes per tour.
  * `stats` (optional, num_tours x 4 int64): passes, pairs evaluated by the reference
@@ -562,9 +564,9 @@ int tspb_batch_survival(const tspb_batch* b, void* stream);
 #define TSPB_BATCH_COORDS 1  /* every item has dist == NULL: distances rebuilt from coordinates */
 #define TSPB_BATCH_GROUPED 2 /* every item's k is a multiple of 4 and its packed table 16-byte aligned */
 /* with GROUPED: every item has rev_off/rev_idx. Best mode keeps the minimum improving key
- * of every row and, after a move with window [bi, bj], recomputes only the rows of the
- * window and the earlier rows with a candidate in it (30 n bytes of shared memory per
- * CTA instead of 16 n); first mode restarts from the move's row after checking the
+ * of every row once the windows are short and, after a move with window [bi, bj], evaluates
+ * only the rows of the window and the entries of earlier rows that point into it (20 n bytes
+ * of shared memory per CTA instead of 10 n); first mode restarts from the move's row after checking the
  * affected entries (as tspb_two_opt with the reverse index). Same results either way. */
 #define TSPB_BATCH_INCREMENTAL 4
 /* best mode, GROUPED, not INCREMENTAL: every row is refined by a two-CTA thread-block

@@ -703,8 +703,8 @@ extern "C" int tspb_batch_two_opt_occupancy(int32_t max_n, int32_t mode, int32_t
   const bool rev = flags & TSPB_BATCH_INCREMENTAL;
   const bool pair = flags & TSPB_BATCH_PAIR;
   if (pair && (rev || mode != TSPB_MODE_BEST)) return 0;
+  if (scan_tour_limit_bytes(max_n, mode, rev) > (size_t)smem_optin() - 2048) return 0;
   const size_t smem = scan_tour_state_bytes(max_n, mode, rev);
-  if (smem > (size_t)smem_optin() - 2048) return 0;
   return mode == TSPB_MODE_BEST ? batch_two_opt_occ_mode<TSPB_MODE_BEST>(threads, smem, rev, pair)
                                 : batch_two_opt_occ_mode<TSPB_MODE_FIRST>(threads, smem, rev, pair);
 }
@@ -726,8 +726,8 @@ extern "C" int tspb_batch_two_opt(const tspb_batch* b, const int32_t* items, int
   if (!items) return TSPB_ERR_ARG;
   if (phase == TSPB_BATCH_PHASE_RESUME && !b->host_elites) return TSPB_ERR_ARG;
   if ((long long)num_items * rows > 0x7fffffffLL || max_n > 65535) return TSPB_ERR_UNSUPPORTED;
+  if (scan_tour_limit_bytes(max_n, mode, rev) > (size_t)smem_optin() - 2048) return TSPB_ERR_UNSUPPORTED;
   const size_t smem = scan_tour_state_bytes(max_n, mode, rev);
-  if (smem > (size_t)smem_optin() - 2048) return TSPB_ERR_UNSUPPORTED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (mode == TSPB_MODE_BEST)
     return batch_two_opt_mode<TSPB_MODE_BEST>(*b, items, num_items, rows, phase, max_iterations, max_n, threads, smem,

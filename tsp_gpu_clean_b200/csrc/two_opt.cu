@@ -339,11 +339,11 @@ static int two_opt_impl(int32_t* tours, int32_t num_tours, int32_t n, const int3
     c.status = status;
     c.ws = reinterpret_cast<unsigned char*>(workspace);
     c.ws_tour_bytes = per;
-    c.arrays_in_smem = per == 0 ? 1 : 0;
+    c.arrays_in_smem = two_opt_scan_in_smem(n, mode) ? 1 : 0;
     c.skip = skip;
     c.budget = watchdog_cycles();
     c.symmetric = symmetric;
-    if (has_rev && mode == TSPB_MODE_FIRST) {  // incremental restart of first mode
+    if (has_rev) {  // incremental restart of first mode, row keys of best mode
       c.rev_off = rev_off;
       c.rev_idx = rev_idx;
     }

@@ -53,7 +53,8 @@ int launch_two_opt_cached(const TwoOptArgs& a, int mode, int threads, cudaStream
 size_t two_opt_cached_tour_bytes(int n, int mode);
 int launch_two_opt_multi(const TwoOptArgs& a, int threads, size_t smem, cudaStream_t st);
 int launch_two_opt_scan(const TwoOptArgs& a, int mode, int threads, cudaStream_t st);
-size_t two_opt_scan_tour_bytes(int n, int mode);
+size_t two_opt_scan_tour_bytes(int n, int mode);  // as the workspace sizes state it
+bool two_opt_scan_in_smem(int n, int mode);
 int carveout_for(int ctas_per_sm, size_t smem_per_cta);
 
 }  // namespace tspb

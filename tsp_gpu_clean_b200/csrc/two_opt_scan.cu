@@ -13,7 +13,7 @@ namespace tspb {
 // SMEM: the tour state lives in shared memory (the compiler then addresses it with
 // shared-memory instructions); otherwise in the per-tour global workspace slice.
 // COUNT: first mode keeps the reference's pair count (launched when stats are requested).
-template <int MODE, int THREADS, int U, int LAYOUT, bool SMEM, bool COUNT>
+template <int MODE, int THREADS, int U, int LAYOUT, bool SMEM, bool COUNT, bool INC>
 __global__ void __launch_bounds__(THREADS, ScanMinBlocks<THREADS>::value) two_opt_scan_kernel(const TwoOptArgs A) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ ScanSmem S;
@@ -39,12 +39,13 @@ __global__ void __launch_bounds__(THREADS, ScanMinBlocks<THREADS>::value) two_op
   T.rev_idx = A.rev_idx;
   T.budget = A.budget;
   T.symmetric = A.symmetric;
-  scan_tour<MODE, THREADS, U, LAYOUT, false, COUNT>(T, S);
+  scan_tour<MODE, THREADS, U, LAYOUT, INC, COUNT>(T, S);
 }
 
-size_t two_opt_scan_tour_bytes(int n, int mode) { return scan_tour_state_bytes(n, mode); }
+size_t two_opt_scan_tour_bytes(int n, int mode) { return scan_tour_limit_bytes(n, mode); }
+bool two_opt_scan_in_smem(int n, int mode) { return scan_tour_state_bytes(n, mode) <= (size_t)smem_optin() - 2048; }
 
-// First mode without stats needs no per-row counts: 16n bytes instead of 20n.
+// First mode without stats needs no per-row counts: 10n bytes instead of 14n.
 static bool scan_counts(const TwoOptArgs& a, int mode) { return mode == TSPB_MODE_FIRST && a.stats != nullptr; }
 
 // Shared-memory carveout (percent of the unified L1/shared array) that holds exactly
@@ -74,23 +75,44 @@ static int carveout_percent(int num_tours, size_t smem_per_cta, int max_ctas_per
   return carveout_for(per_sm, smem_per_cta);
 }
 
+// The grouped layout loads four packed words at once: k % 4 == 0 and a 16-byte aligned table.
+static bool scan_grouped(const TwoOptArgs& a) {
+  return a.cand_packed && a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(a.cand_packed) % 16) == 0;
+}
+
+// Best mode with row keys: where the reverse index is given, the larger state still fits in
+// shared memory and a full rescan takes a CTA eight rounds or more. Below that a pass is a
+// chain of latencies and the keys' extra barriers lose: 64 tours of 200 cities (2 rounds) 0.70
+// ms without keys, 0.98 with; 1 of 500 (5 rounds) 2.55 and 2.79; 8 of 2000 (20 rounds) 30.8
+// and 22.9; 1024 of 1000 (39 rounds) 45.1 and 29.4.
+static bool scan_row_keys(const TwoOptArgs& a, int mode, int threads) {
+  return mode == TSPB_MODE_BEST && scan_grouped(a) && a.rev_off && a.rev_idx && a.k <= 32 &&
+         (long long)(a.n - 2) * (a.k / 4) >= 8LL * threads &&
+         scan_tour_state_bytes(a.n, mode, true, a.stats != nullptr) <= (size_t)smem_optin() - 2048;
+}
+
 template <int MODE, int THREADS, int U>
 static int launch_scan(const TwoOptArgs& a, size_t smem, cudaStream_t st) {
-  // the grouped layout loads U packed words at once: k % U == 0 and a U*4-byte aligned table
+  using Kern = void (*)(const TwoOptArgs);
   const bool aligned = (reinterpret_cast<uintptr_t>(a.cand_packed) % (U * sizeof(uint32_t))) == 0;
   const int layout = a.cand_packed ? (a.k % U == 0 && aligned ? SCAN_GROUPED : SCAN_PACKED) : SCAN_PLAIN;
-  // best mode has no per-row counts: one instance serves both
+  // best mode without row keys has no per-row counts: one instance serves both
   constexpr bool CAN_SKIP = MODE == TSPB_MODE_FIRST;
-  auto pick = [&](auto smem_tag, auto count_tag) {
+  auto pick = [&](auto smem_tag, auto count_tag) -> Kern {
     constexpr bool SM = decltype(smem_tag)::value;
     constexpr bool CT = decltype(count_tag)::value || !CAN_SKIP;
-    return layout == SCAN_GROUPED  ? two_opt_scan_kernel<MODE, THREADS, U, SCAN_GROUPED, SM, CT>
-           : layout == SCAN_PACKED ? two_opt_scan_kernel<MODE, THREADS, U, SCAN_PACKED, SM, CT>
-                                   : two_opt_scan_kernel<MODE, THREADS, U, SCAN_PLAIN, SM, CT>;
+    return layout == SCAN_GROUPED  ? two_opt_scan_kernel<MODE, THREADS, U, SCAN_GROUPED, SM, CT, false>
+           : layout == SCAN_PACKED ? two_opt_scan_kernel<MODE, THREADS, U, SCAN_PACKED, SM, CT, false>
+                                   : two_opt_scan_kernel<MODE, THREADS, U, SCAN_PLAIN, SM, CT, false>;
   };
   const bool count = scan_counts(a, MODE);
-  auto kern = a.arrays_in_smem ? (count ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
+  Kern kern = a.arrays_in_smem ? (count ? pick(std::true_type{}, std::true_type{}) : pick(std::true_type{}, std::false_type{}))
                                : (count ? pick(std::false_type{}, std::true_type{}) : pick(std::false_type{}, std::false_type{}));
+  if constexpr (MODE == TSPB_MODE_BEST && U == 4) {
+    if (scan_row_keys(a, MODE, THREADS))
+      kern = a.stats ? two_opt_scan_kernel<MODE, THREADS, U, SCAN_GROUPED, true, true, true>
+                     : two_opt_scan_kernel<MODE, THREADS, U, SCAN_GROUPED, true, false, true>;
+  }
   if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int pct = carveout_percent(a.num_tours, smem, ScanMinBlocks<THREADS>::value);
   if (pct > 0) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
@@ -103,16 +125,18 @@ static int launch_scan_mode(const TwoOptArgs& a, int threads, size_t smem, cudaS
   switch (threads) {
     case 64: return launch_scan<MODE, 64, 4>(a, smem, st);
     case 128: return launch_scan<MODE, 128, 4>(a, smem, st);
-    case 512: {  // four entries per thread in flight only where the grouped layout applies
-      const bool grouped = a.cand_packed && a.k % 4 == 0 && (reinterpret_cast<uintptr_t>(a.cand_packed) % 16) == 0;
-      return grouped ? launch_scan<MODE, 512, 4>(a, smem, st) : launch_scan<MODE, 512, 2>(a, smem, st);
-    }
+    case 512:  // four entries per thread in flight only where the grouped layout applies
+      return scan_grouped(a) ? launch_scan<MODE, 512, 4>(a, smem, st) : launch_scan<MODE, 512, 2>(a, smem, st);
     default: return launch_scan<MODE, 256, 4>(a, smem, st);
   }
 }
 
 int launch_two_opt_scan(const TwoOptArgs& a, int mode, int threads, cudaStream_t st) {
-  const size_t smem = a.arrays_in_smem ? scan_tour_state_bytes(a.n, mode, false, scan_counts(a, mode)) : 0;
+  if (threads != 64 && threads != 128 && threads != 512) threads = 256;
+  const bool keys = scan_row_keys(a, mode, threads);
+  const size_t smem = keys                ? scan_tour_state_bytes(a.n, mode, true, a.stats != nullptr)
+                      : a.arrays_in_smem ? scan_tour_state_bytes(a.n, mode, false, scan_counts(a, mode))
+                                         : 0;
   if (mode == TSPB_MODE_BEST) return launch_scan_mode<TSPB_MODE_BEST>(a, threads, smem, st);
   return launch_scan_mode<TSPB_MODE_FIRST>(a, threads, smem, st);
 }

@@ -145,7 +145,7 @@ class LocalSearchB200TourTwoOpt(StrategyBase):
     cand_dist = tabs.cand_dist if tabs is not None else None
     cached = tabs is not None and self.kernel == "cached"
     packed = tabs.packed if tabs is not None and self.kernel == "scan" else None
-    use_rev = cached or (packed is not None and self.mode == "first" and self.incremental_first)
+    use_rev = cached or (packed is not None and (self.mode != "first" or self.incremental_first))
     rev_off = tabs.rev_off if use_rev else None
     rev_idx = tabs.rev_idx if use_rev else None
     native.call(
