@@ -302,11 +302,66 @@ __global__ void validate_perm_kernel(const int32_t* __restrict__ tours, int n, i
   if (threadIdx.x == 0) bad_out[r] = bad;
 }
 
-__global__ void euc2d_matrix_kernel(const double2* __restrict__ coords, int n, int32_t* __restrict__ dist, long long stride) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int a = blockIdx.y;
-  if (c >= n) return;
-  dist[(long long)a * stride + c] = a == c ? 0 : euc2d(__ldg(coords + a), __ldg(coords + c));
+// EUC_2D matrix, four columns of one row per thread and step (16-byte stores where the rows
+// allow them).
+//
+// What bounds it: writing the 4 n^2 bytes. The correctly rounded FP64 root of every entry did
+// before (n = 10,000: 222 us; 115 in this form, 61 for the bytes at copy speed), so an entry takes it
+// only when FP32 cannot settle the rounding: d is computed in FP32 with the error bound below,
+// and accepted when its distance from the nearest integer leaves half a unit minus that bound.
+//   coordinates: rounding each to FP32 moves it by at most 2^-24 |x|, the difference adds
+//   2^-24 of its value, so |error of dx| + |error of dy| <= 2^-24 (mag_a + mag_b) + 2^-24
+//   (|dx| + |dy|), with mag = |x| + |y|; the root of the sum of squares moves by no more than
+//   that (the triangle inequality), and the squares, their sum and sqrt.approx (2^-23) by less
+//   than 2^-21 d. 2^-23 (mag_a + mag_b) + 2^-20 d bounds all of it, d + 0.5 included.
+// 1000 x 1000 squares send about one entry in 2,000 to the FP64 form.
+__global__ void __launch_bounds__(256) euc2d_matrix_kernel(const double2* __restrict__ coords, int n,
+                                                           int32_t* __restrict__ dist, long long stride, int rows, int wide) {
+  const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (c0 >= n) return;
+  float2 p[4];
+  float mag[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double2 v = __ldg(coords + (c0 + q < n ? c0 + q : n - 1));
+    p[q] = make_float2((float)v.x, (float)v.y);
+    mag[q] = 0x1p-23f * (fabsf(p[q].x) + fabsf(p[q].y));
+  }
+  const int a_end = min((int)(blockIdx.y + 1) * rows, n);
+  for (int a = blockIdx.y * rows; a < a_end; ++a) {
+    const double2 va = __ldg(coords + a);
+    const float2 pa = make_float2((float)va.x, (float)va.y);
+    const float mag_a = 0x1p-23f * (fabsf(pa.x) + fabsf(pa.y));
+    int d[4];
+    bool redo = false;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float dx = pa.x - p[q].x, dy = pa.y - p[q].y;
+      float r;
+      asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(fmaf(dx, dx, dy * dy)));
+      const float err = mag_a + mag[q] + 0x1p-20f * r;
+      // nearest integer by adding 1.5 * 2^23 (no conversion: those share the root's unit); r
+      // minus it is exact. Roots of 2^19 and more, infinities and NaN fail the test.
+      const float m = __fadd_rn(r, 12582912.0f);
+      d[q] = __float_as_int(m) - __float_as_int(12582912.0f);
+      redo |= !(fabsf(__fsub_rn(r, __fsub_rn(m, 12582912.0f))) < 0.5f - err);
+    }
+    if (redo) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) d[q] = euc2d(va, __ldg(coords + (c0 + q < n ? c0 + q : n - 1)));
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c0 + q == a) d[q] = 0;
+    int32_t* row = dist + (long long)a * stride + c0;
+    if (wide && c0 + 4 <= n) {
+      *reinterpret_cast<int4*>(row) = make_int4(d[0], d[1], d[2], d[3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (c0 + q < n) row[q] = d[q];
+    }
+  }
 }
 
 __global__ void cand_dist_kernel(const int32_t* __restrict__ cand, int n, int k, DistSrc ds, int32_t* __restrict__ out) {
@@ -447,9 +502,15 @@ extern "C" int tspb_euc2d_matrix(const double* coords, int32_t n, int32_t* dist,
   if (n == 0) return TSPB_OK;
   if (!coords || !dist) return TSPB_ERR_ARG;
   if (n > 65535) return TSPB_ERR_UNSUPPORTED;
-  dim3 grid((n + 255) / 256, n);
+  // up to eight rows per thread (the columns' coordinates are read once), fewer where that
+  // would leave SMs without a CTA
+  const int strips = (n + 1023) / 1024;
+  int rows = 8;
+  while (rows > 1 && (long long)strips * (n / rows) < 2 * 148) rows >>= 1;
+  const dim3 grid(strips, (n + rows - 1) / rows);
+  const int wide = dist_stride % 4 == 0 && reinterpret_cast<uintptr_t>(dist) % 16 == 0;
   euc2d_matrix_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const double2*>(coords), n,
-                                                                                  dist, dist_stride);
+                                                                                  dist, dist_stride, rows, wide);
   return tspb_launch_status();
 }
 
