@@ -13,8 +13,9 @@
 //     the window [i, j] touches no accepted window (:491-563);
 //   - at most max_iterations passes, stopping at the first pass without a move (:565-595).
 //
-// This file holds the exhaustive best / first scans and the C entry points; the candidate
-// scans are in two_opt_scan.cuh and two_opt_cached.cu, multi_move in two_opt_multi.cu.
+// This file holds the C entry points and the general exhaustive best / first scans (distances
+// rebuilt from coordinates, or tours too long for two_opt_all.cu); the candidate scans are in
+// two_opt_scan.cuh and two_opt_cached.cu, multi_move in two_opt_multi.cu.
 //
 // Device layout per tour: tour and edge (d(tour[p], tour[p+1])) as int32 arrays in shared
 // memory when they fit, else in the caller's global workspace.
@@ -401,6 +402,9 @@ static int two_opt_impl(int32_t* tours, int32_t num_tours, int32_t n, const int3
   a.budget = watchdog_cycles();
   a.cand_packed = use_cand ? cand_packed : nullptr;
   if (mode == TSPB_MODE_MULTI_MOVE) return launch_two_opt_multi(a, threads, L.smem_bytes, st);
+  a.symmetric = symmetric;
+  int rc = TSPB_OK;
+  if (launch_two_opt_all(a, mode, threads, st, &rc)) return rc;
   return mode == TSPB_MODE_BEST ? launch<TSPB_MODE_BEST>(a, threads, L.smem_bytes, st)
                                 : launch<TSPB_MODE_FIRST>(a, threads, L.smem_bytes, st);
 }

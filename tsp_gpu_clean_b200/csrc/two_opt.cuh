@@ -26,7 +26,7 @@ struct TwoOptArgs {
   const uint32_t* cand_packed;  // scan kernel: c | d(a, c) << 16 per entry (optional)
   const int32_t* skip;          // optional device flag: non-zero makes the launch a no-op
   long long budget;             // watchdog: SM cycles a tour may run (watchdog_cycles())
-  int symmetric;                // scan kernel: symmetric distances (TSPB_MODE_SYMMETRIC)
+  int symmetric;                // symmetric distances (TSPB_MODE_SYMMETRIC)
 };
 
 // Order-preserving u64 key: negative int32 gain in the high word, scan index low.
@@ -51,6 +51,7 @@ int device_attr(cudaDeviceAttr attr);
 size_t align256(size_t v);
 int launch_two_opt_cached(const TwoOptArgs& a, int mode, int threads, cudaStream_t st);
 size_t two_opt_cached_tour_bytes(int n, int mode);
+bool launch_two_opt_all(const TwoOptArgs& a, int mode, int threads, cudaStream_t st, int* status);
 int launch_two_opt_multi(const TwoOptArgs& a, int threads, size_t smem, cudaStream_t st);
 int launch_two_opt_scan(const TwoOptArgs& a, int mode, int threads, cudaStream_t st);
 size_t two_opt_scan_tour_bytes(int n, int mode);  // as the workspace sizes state it
