@@ -347,7 +347,8 @@ int tspb_three_opt_grid_threads(int32_t threads_per_block, int32_t n);
  * cand_packed (optional): the same as c | d << 16 words (tspb_candidate_pack, no overflow),
  * read four at a time when k % 4 == 0 and the table is 16-byte aligned;
  * distances from `dist` (n x dist_stride) or rebuilt from EUC_2D `coords`. One CTA per
- * tour (persistent), `threads` 128, 256 or 512, 16 n bytes of shared memory
+ * tour (persistent), `threads` 128, 256 or 512 (taken wider where tours leave SMs idle),
+ * 16 n bytes of shared memory
  * (n <= tspb_or_opt_max_n()). n < 3: nothing to do. stats (optional): [tours][3] passes,
  * moves, valid entries evaluated.
  */
