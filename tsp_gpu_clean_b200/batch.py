@@ -353,9 +353,8 @@ class FusedBatchSolver:
 
   @staticmethod
   def _survival_launches() -> int:
-    """Kernels of tspb_batch_survival: the rank (with the elite-edge tie check), then the
-    survivor gather."""
-    return 2
+    """Kernels of tspb_batch_survival: rank, elite-edge tie check and survivor copy in one."""
+    return 1
 
   def _launches_per_replay(self, resume: bool = False) -> int:
     nb = len(self.buckets)

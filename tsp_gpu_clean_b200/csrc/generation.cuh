@@ -22,21 +22,45 @@ struct GenTapeSlice {
   const int32_t* inv_b;  // [P]
 };
 
+// The first contestant with the smallest fitness, by a whole warp: a lane per contestant, so
+// that the tape words and then the fitness values are read together instead of one after
+// another. Entries outside 0..pop-1 count as absent (the first of them as row 0).
 __device__ __forceinline__ int tournament_winner(const double* fit, const int32_t* c, int kt, int pop) {
-  int best = c[0];
-  if ((unsigned)best >= (unsigned)pop) best = 0;
-  double bf = fit[best];
-  for (int q = 1; q < kt; ++q) {
-    const int v = c[q];
-    if ((unsigned)v >= (unsigned)pop) continue;
+  const int lane = threadIdx.x & 31;
+  int at = kt, best = 0;
+  double bf = __longlong_as_double(0x7ff0000000000000LL);
+  for (int q = lane; q < kt; q += 32) {
+    int v = c[q];
+    if ((unsigned)v >= (unsigned)pop) {
+      if (q != 0) continue;
+      v = 0;
+    }
     const double f = fit[v];
-    if (f < bf) {
+    if (q == 0 || f < bf || at == kt) {
       bf = f;
       best = v;
+      at = q;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double of = __shfl_xor_sync(FULL, bf, o);
+    const int oa = __shfl_xor_sync(FULL, at, o), ob = __shfl_xor_sync(FULL, best, o);
+    if (oa < kt && (at == kt || of < bf || (of == bf && oa < at))) {
+      bf = of;
+      at = oa;
+      best = ob;
     }
   }
   return best;
 }
+
+// What bounds a child is a chain of L2 latencies (control block, tape, fitness, parents,
+// distances), so the rows and the distances are read OFFSPRING_AHEAD values a thread at a
+// time, and PMX's chains walk p1's segment in shared memory: 512 children of 1000 cities 8.5 us
+// (11.1 one value at a time); buckets of 128 runs of 64 rows beside one another 22.8 us a
+// launch (32.7).
+constexpr int OFFSPRING_AHEAD = 4;
 
 // Shared memory of offspring_row: inv_p2[n], child[n] ints and the in-segment bitmap.
 __host__ __device__ inline size_t offspring_smem_bytes(int n) {
@@ -127,9 +151,10 @@ __device__ __forceinline__ void offspring_row(const int32_t* __restrict__ pop, c
   const int pairs = P >> 1;
   const int q = row >> 1, h = row & 1;
   const bool paired = row < 2 * pairs;
-  if (tid < 2) {
-    const int sel = paired ? 2 * q + (tid == 0 ? h : 1 - h) : row;
-    w[tid] = tournament_winner(fit, tape.tourn + (long long)sel * kt, kt, P);
+  for (int side = tid >> 5; side < 2; side += T >> 5) {
+    const int sel = paired ? 2 * q + (side == 0 ? h : 1 - h) : row;
+    const int won = tournament_winner(fit, tape.tourn + (long long)sel * kt, kt, P);
+    if ((tid & 31) == 0) w[side] = won;
   }
   __syncthreads();
   const int32_t* p1 = pop + (long long)w[0] * n;
@@ -161,15 +186,25 @@ __device__ __forceinline__ void offspring_row(const int32_t* __restrict__ pop, c
       c2 = tmp;
     }
     const int words = (n + 31) >> 5;
-    for (int p = tid; p < n; p += T) child[p] = -1;
     for (int wd = tid; wd < words; wd += T) in_seg[wd] = 0u;
     __syncthreads();
-    for (int p = tid; p < n; p += T) {
-      inv_p2[__ldg(p2 + p)] = p;
-      if (p >= c1 && p <= c2) {
-        const int v1 = __ldg(p1 + p);
-        child[p] = v1;
-        atomicOr(&in_seg[v1 >> 5], 1u << (v1 & 31));
+    // p1's segment, p2 outside it until a chain below ends there
+    for (int p0 = tid; p0 < n; p0 += OFFSPRING_AHEAD * T) {
+      int v1[OFFSPRING_AHEAD], v2[OFFSPRING_AHEAD];
+#pragma unroll
+      for (int u = 0; u < OFFSPRING_AHEAD; ++u) {
+        const int p = p0 + u * T;
+        v1[u] = (int)load_nc_if(p >= c1 && p <= c2, p1 + p);
+        v2[u] = (int)load_nc_if(p < n, p2 + p);
+      }
+#pragma unroll
+      for (int u = 0; u < OFFSPRING_AHEAD; ++u) {
+        const int p = p0 + u * T;
+        if (p >= n) break;
+        const bool seg = p >= c1 && p <= c2;
+        inv_p2[v2[u]] = p;
+        child[p] = seg ? v1[u] : v2[u];
+        if (seg) atomicOr(&in_seg[v1[u] >> 5], 1u << (v1[u] & 31));
       }
     }
     __syncthreads();
@@ -179,14 +214,11 @@ __device__ __forceinline__ void offspring_row(const int32_t* __restrict__ pop, c
       if (in_seg[val >> 5] & (1u << (val & 31))) continue;
       int pos = idx, steps = 0;
       while (pos >= c1 && pos <= c2 && steps <= seg_len) {
-        pos = inv_p2[__ldg(p1 + pos)];
+        pos = inv_p2[child[pos]];  // p1's gene: nothing writes inside the segment now
         ++steps;
       }
       if (pos < c1 || pos > c2) child[pos] = val;
     }
-    __syncthreads();
-    for (int p = tid; p < n; p += T)
-      if (child[p] == -1) child[p] = __ldg(p2 + p);
   }
   __syncthreads();
   // mutation of this child
@@ -212,13 +244,26 @@ __device__ __forceinline__ void offspring_row(const int32_t* __restrict__ pop, c
   // write out and reduce the closed-tour length (exact int64, one float64 at the end)
   long long acc = 0;
   int diff1 = 0, diff2 = 0;
-  for (int p = tid; p < n; p += T) {
-    const int v = child[p];
-    off_row[p] = v;
-    acc += ds(v, child[p + 1 == n ? 0 : p + 1]);
-    if (origin) {
-      diff1 |= v != __ldg(p1 + p);
-      diff2 |= v != __ldg(p2 + p);
+  for (int p0 = tid; p0 < n; p0 += OFFSPRING_AHEAD * T) {
+    int d[OFFSPRING_AHEAD], v[OFFSPRING_AHEAD], g1[OFFSPRING_AHEAD], g2[OFFSPRING_AHEAD];
+#pragma unroll
+    for (int u = 0; u < OFFSPRING_AHEAD; ++u) {
+      const int p = p0 + u * T;
+      const bool in = p < n;
+      v[u] = in ? child[p] : 0;
+      const int next = in ? child[p + 1 == n ? 0 : p + 1] : 0;
+      d[u] = ds.dist != nullptr ? load_cg_if(in, ds.dist + (long long)v[u] * ds.stride + next) : (in ? ds(v[u], next) : 0);
+      g1[u] = (int)load_nc_if(in && origin, p1 + p);
+      g2[u] = (int)load_nc_if(in && origin, p2 + p);
+      if (in) off_row[p] = v[u];
+    }
+#pragma unroll
+    for (int u = 0; u < OFFSPRING_AHEAD; ++u) {
+      acc += d[u];
+      if (p0 + u * T < n) {
+        diff1 |= v[u] != g1[u];
+        diff2 |= v[u] != g2[u];
+      }
     }
   }
   acc = block_sum(acc, red);
