@@ -162,6 +162,24 @@ def elite_rows(fitness: np.ndarray, elite: int) -> np.ndarray:
   return np.argsort(fitness, axis=1)[:, :elite].astype(np.int32)
 
 
+def _ctl_offset(runs: int, elite: int) -> int:
+  return -(-4 * runs * max(elite, 1) // 16) * 16
+
+
+def _fit_offset(runs: int, elite: int) -> int:
+  return _ctl_offset(runs, elite) + 16 * runs
+
+
+def _exchange_buffer(runs: int, P: int, elite: int, device):
+  """Zeroed bytes on `device` (None: pinned host memory) and their views: host elites
+  (runs, elite), control blocks (runs, 4), fitness (2, runs, P)."""
+  a, b = _ctl_offset(runs, elite), _fit_offset(runs, elite)
+  e = max(elite, 1)
+  buf = torch.zeros(b + 16 * runs * P, dtype=torch.uint8, device=device or "cpu", pin_memory=device is None)
+  return buf, (buf[: 4 * runs * e].view(torch.int32).view(runs, e), buf[a:b].view(torch.int32).view(runs, 4),
+               buf[b:].view(torch.float64).view(2, runs, P))
+
+
 class FusedBatchSolver:
   def __init__(self, population_size: int = 64, mutation_rate: float = 0.05, tournament_k: int = 5, nn_k: int = 5,
                local_search: LocalSearchConfig | None = None, elite_count: int = 8, post_init: bool = True,
@@ -649,15 +667,17 @@ class FusedBatchSolver:
     dev = "cuda"
     self.pop = [torch.empty(P * total, dtype=torch.int32, device=dev) for _ in range(2)]
     self.off = torch.empty(P * total, dtype=torch.int32, device=dev)
-    self.fit = [torch.zeros((self.I, P), dtype=torch.float64, device=dev) for _ in range(2)]
     self.off_fit = torch.zeros((self.I, P), dtype=torch.float64, device=dev)
     self.order = torch.zeros((self.I, P), dtype=torch.int32, device=dev)
-    self.ctl = torch.zeros((self.I, 4), dtype=torch.int32, device=dev)
     self.best_cost = torch.zeros(self.I, dtype=torch.float64, device=dev)
     self.best_tour = torch.zeros(total, dtype=torch.int32, device=dev)
     self.history = torch.zeros((self.I, G + 1), dtype=torch.float64, device=dev)
     self.ties = torch.zeros((self.I, max(G, 1)), dtype=torch.int32, device=dev)
-    self.host_elites = torch.zeros((self.I, max(self.elite, 1)), dtype=torch.int32, device=dev)
+    # what a host check moves, in one buffer so that each direction is one copy: the host's
+    # elites | control blocks | both fitness buffers; the checks read the last two and answer
+    # with the first two
+    exchange, views = _exchange_buffer(self.I, P, self.elite, dev)
+    self.host_elites, self.ctl, self.fit = views[0], views[1], [views[2][0], views[2][1]]
     self.ls_status = torch.zeros((self.I, P), dtype=torch.int32, device=dev)
     self.ls_stats = torch.zeros((self.I, P, 4), dtype=torch.int64, device=dev)
     self.clean = [torch.zeros((self.I, P), dtype=torch.uint8, device=dev) for _ in range(2)]
@@ -780,22 +800,21 @@ class FusedBatchSolver:
     ev_start = torch.cuda.Event(enable_timing=True)
     ev_end = torch.cuda.Event(enable_timing=True)
     ev_start.record()
-    ctl_host = torch.empty((self.I, 4), dtype=torch.int32, pin_memory=True)
-    # each round's snapshot also carries both fitness buffers, so a paused run's fitness
-    # needs no further read; the host's answers go back through pinned buffers without a
-    # sync (the next round's snapshot is ordered after them)
-    fit_host = torch.empty((2, self.I, P), dtype=torch.float64, pin_memory=True)
-    ctl_up = torch.empty((self.I, 4), dtype=torch.int32, pin_memory=True)
-    he_up = torch.zeros((self.I, max(self.elite, 1)), dtype=torch.int32, pin_memory=True)
-    he_host = he_up.numpy()
+    # each check's snapshot carries both fitness buffers, so a paused run's fitness needs no
+    # further read; the host's answers go back through pinned memory without a sync (the next
+    # check's snapshot is ordered after them)
+    snap, (_, ctl_host, fit_host) = _exchange_buffer(self.I, P, self.elite, None)
+    answer, (he_up, ctl_up, _) = _exchange_buffer(self.I, 0, self.elite, None)
+    he_host, c, fits_host = he_up.numpy(), ctl_host.numpy(), fit_host.numpy()
+    snap_from, answer_to = _ctl_offset(self.I, self.elite), _fit_offset(self.I, self.elite)
+    stream = torch.cuda.current_stream()
     ready = torch.cuda.Event()
     host_elite_gens = np.zeros(self.I, dtype=np.int64)
-    live = (native.TSPB_BATCH_RUN, native.TSPB_BATCH_PAUSED, native.TSPB_BATCH_RESUME)
     # Every round (replays, then one host check) advances each live run by a generation
     # or leaves it paused for the host, who resumes it before the next round.
     rounds, max_rounds = 0, 2 * G + 2
     chunk, remaining = min(self.chunk, max(G, 1)), G
-    c = None
+    alive = np.zeros(self.I, dtype=bool)
     need_resume = False  # runs the host resumed wait for the next replay's RESUME phase
     while G > 0 and rounds < max_rounds:
       for q in range(max(1, min(chunk, remaining))):
@@ -809,28 +828,23 @@ class FusedBatchSolver:
           self._generation(resume)
         self.replays += 1
       rounds += 1
-      ctl_host.copy_(self.ctl, non_blocking=True)
-      fit_host[0].copy_(self.fit[0], non_blocking=True)
-      fit_host[1].copy_(self.fit[1], non_blocking=True)
-      ready.record()
+      snap[snap_from:].copy_(exchange[snap_from:], non_blocking=True)
+      ready.record(stream)
       ready.synchronize()
-      c = ctl_host.numpy()
-      paused = np.nonzero(c[:, 1] == native.TSPB_BATCH_PAUSED)[0]
+      state = c[:, 1]
+      paused = np.flatnonzero(state == native.TSPB_BATCH_PAUSED)
       if paused.size:
         parity = (c[paused, 0] + 1) & 1
-        fits = fit_host.numpy()[parity, paused]
-        he_host[paused] = elite_rows(fits, self.elite)  # pipeline_steps.py:163
-        self.host_elites.copy_(he_up, non_blocking=True)
-        c = c.copy()
-        c[paused, 1] = native.TSPB_BATCH_RESUME
+        he_host[paused] = elite_rows(fits_host[parity, paused], self.elite)  # pipeline_steps.py:163
+        state[paused] = native.TSPB_BATCH_RESUME
         ctl_up.numpy()[...] = c
-        self.ctl.copy_(ctl_up, non_blocking=True)
+        exchange[:answer_to].copy_(answer[:answer_to], non_blocking=True)
         host_elite_gens[paused] += 1
         chunk = max(1, chunk // 2)
       else:
         chunk = min(2 * chunk, self.chunk)
       need_resume = bool(paused.size)
-      alive = np.isin(c[:, 1], live)
+      alive = (state == native.TSPB_BATCH_RUN) | (state == native.TSPB_BATCH_RESUME)
       if not alive.any():
         break
       remaining = G - int(c[alive, 0].min())
@@ -838,7 +852,7 @@ class FusedBatchSolver:
     torch.cuda.synchronize()
     t_end = time.perf_counter()
     loop_ms = ev_start.elapsed_time(ev_end)
-    if G > 0 and c is not None and np.isin(c[:, 1], live).any():
+    if alive.any():
       raise RuntimeError("batch GA did not finish within its round bound")
     if int(self.ls_status.max().item()) != 0:
       raise RuntimeError(f"2-opt kernel reported status {int(self.ls_status.max().item())} inside the batch GA")
