@@ -23,25 +23,9 @@ constexpr unsigned FULL = 0xffffffffu;
 // TSPLIB EUC_2D from FP64 coordinates with one IEEE rounding per operation, in the
 // order NumPy evaluates `(sqrt(sum(diff * diff)) + 0.5).astype(int64)`: two products,
 // one sum, a correctly rounded square root, +0.5, truncation. No contraction to FMA.
-//
-// The root is about 45 FP64 instructions; it is taken only where FP32 cannot settle the
-// rounding. dx and dy are exact to 2^-53 and rounded once to FP32, so the approximate root r
-// is within 2^-22 r of the true one (two roundings of each square and its sum, halved by the
-// root, and sqrt.approx's 2^-23); where the nearest integer m leaves more than 2^-20 r to both
-// half-integers, m is the result of both forms. Distances of a few hundred send about one pair
-// in 1,000 to the FP64 form; roots of 2^19 and more, infinities and NaN always go there. The
-// 2-opt of batch runs on coordinates (1025 to 4096 cities): 163 -> 155 us a launch, 117 -> 112
-// by CTA pairs.
 __device__ __forceinline__ int euc2d(const double2 p, const double2 q) {
   const double dx = __dsub_rn(p.x, q.x);
   const double dy = __dsub_rn(p.y, q.y);
-  const float fx = (float)dx, fy = (float)dy;
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(fmaf(fx, fx, fy * fy)));
-  // nearest integer by adding 1.5 * 2^23; r minus it is exact
-  const float m = __fadd_rn(r, 12582912.0f);
-  if (fabsf(__fsub_rn(r, __fsub_rn(m, 12582912.0f))) < 0.5f - 0x1p-20f * r)
-    return __float_as_int(m) - __float_as_int(12582912.0f);
   const double s = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
   return (int)(long long)__dadd_rn(__dsqrt_rn(s), 0.5);
 }
