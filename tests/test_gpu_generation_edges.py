@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("scale", [1.0, 37.0, 1000.0, 3.0e5, 4.0e6, 1.0e8])
 def test_euc2d_at_half_integers(scale):
   """Distances on, one ulp below and one ulp above m + 0.5, and random ones, from
-  coordinates (no matrix): the FP32 form may only answer where the FP64 form agrees."""
+  coordinates (no matrix), against NumPy's rounding."""
   import torch
 
   from tsp_gpu_clean_b200 import native
