@@ -281,10 +281,11 @@ __device__ __forceinline__ void scan_tour(const ScanTour T, ScanSmem& S) {
   bool converged = false;  // the last pass found no improving move: a local optimum
   const long long t_start = clock64();
   const bool incremental = MODE == TSPB_MODE_FIRST && T.rev_off != nullptr && T.rev_idx != nullptr;
-  // entry e = a * k + r of the reverse index -> a, as a multiply-high by ceil(2^32 / k):
-  // exact for every e < n k when n k k < 2^32 (else a plain division)
+  // e / k of an entry e = a * k + r, as a multiply-high by ceil(2^32 / k): exact for every
+  // e < n k when n k k < 2^32 and the reciprocal itself fits 32 bits, which k = 1 does not
+  // (else a plain division)
   const unsigned kmag = (unsigned)(((1ull << 32) + (unsigned)k - 1) / (unsigned)k);
-  const bool kmag_exact = (unsigned long long)n * (unsigned)k * (unsigned)k < (1ull << 32);
+  const bool kmag_exact = k > 1 && (unsigned long long)n * (unsigned)k * (unsigned)k < (1ull << 32);
   auto entry_node = [&](int e) -> int {
     return kmag_exact ? (int)__umulhi((unsigned)e, kmag) : e / k;
   };
