@@ -151,8 +151,9 @@ __global__ void __launch_bounds__(1024) two_opt_multi_kernel(const TwoOptArgs A)
   const long long exh_total = (long long)(n - 3) + (long long)(n - 3) * (n - 2) / 2;
   const unsigned div = CAND ? (unsigned)k : (unsigned)n;  // scan index = i * div + column
   // i of a scan index by multiply-high with ceil(2^32 / div): exact while index * div < 2^32
+  // and the reciprocal itself fits 32 bits, which div = 1 does not
   const unsigned mag = (unsigned)(((1ull << 32) + div - 1) / div);
-  const bool mag_exact = (unsigned long long)n * div * div < (1ull << 32);
+  const bool mag_exact = div > 1 && (unsigned long long)n * div * div < (1ull << 32);
   auto row_of = [&](unsigned idx) -> int { return (int)(mag_exact ? __umulhi(idx, mag) : idx / div); };
   // second position of pair idx of row i; used while row i touches no accepted window
   auto col_of = [&](unsigned idx, int i) -> int {
