@@ -36,7 +36,8 @@ namespace {
 
 constexpr int kUnitRows = 8;     // rows per warp unit
 constexpr int kSlice = 31;       // second positions of a warp's pairs
-constexpr int kAllThreads = 512;  // at most: a unit's rows and minima take about 100 registers
+// Threads of a CTA and of an SM at most: a unit's rows and minima take some 120 registers.
+constexpr int kAllThreads = 512;
 constexpr long long kCpuBlock = 1LL << 18;  // exhaustive pairs per CPU block (two_opt.py:155)
 
 struct AllSmem {
@@ -446,23 +447,30 @@ __global__ void __launch_bounds__(kAllThreads) two_opt_all_kernel(const TwoOptAr
   }
 }
 
-// Launches the kernel when its rows fit in shared memory; false: the caller takes the general
-// one (distances rebuilt from coordinates, or rows too long for tiles of kUnitRows).
+// Launches the kernel when its rows fit in shared memory and the run is long enough for them;
+// false: the caller takes the general one (distances rebuilt from coordinates, rows too long
+// for tiles of kUnitRows, tours or runs so short that a pass costs less than setting up for it).
 bool launch_two_opt_all(const TwoOptArgs& a, int mode, int threads, cudaStream_t st, int* status) {
+  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
+  const int sm_bytes = device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
+  if (sms <= 0 || sm_bytes <= 0) return false;
   // Below 64 cities a pass is a few hundred cycles and the general kernel's fewer barriers win:
-  // 100 tours of 50 cities 0.25 ms there and 0.30 here, of 70 cities 0.46 and 0.38.
-  if (a.ds.dist == nullptr || a.n < 64) return false;
+  // 100 tours of 50 cities 0.25 ms there and 0.30 here, of 70 cities 0.46 and 0.38. So they do
+  // for the shortest runs: ten passes of 148 tours of 64 cities 0.14 and 0.16 ms, one pass of
+  // 5000 tours of 130 cities 0.25 and 0.32.
+  if (a.ds.dist == nullptr || a.n < 64 || (a.n < 72 && a.max_iter <= 16)) return false;
+  if (a.num_tours > sms && mode == TSPB_MODE_BEST && a.max_iter == 1 && a.n < 300) return false;
   threads = std::min(threads, kAllThreads);
   const long long pitch = (a.n + 3) & ~3;
   const long long slices = (a.n + kSlice - 1) / kSlice;
   // tour, edges, and best's row keys and two tiles of keys by slice
   auto state = [&](long long tile) { return (mode == TSPB_MODE_BEST ? 16LL * a.n + 16 * tile * slices : 8LL * a.n) + 16; };
-  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
-  const int sm_bytes = device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
-  if (sms <= 0 || sm_bytes <= 0) return false;
-  int resident = std::max(1, std::min((a.num_tours + sms - 1) / sms, 2048 / threads));
+  // CTAs an SM: as many as there are tours for and registers hold. (Shared memory split for more
+  // of them than registers hold leaves small tiles: best, ten passes of 5000 tours of 90 cities
+  // 1.71 ms that way and 0.81 this, 0.93 in the general kernel.)
+  int resident = std::max(1, std::min((a.num_tours + sms - 1) / sms, kAllThreads / threads));
   int tile = 0, whole = 0;
-  for (; resident >= 1 && tile == 0; --resident) {
+  while (true) {
     const long long share = std::min<long long>(sm_bytes / resident - 1024, smem_optin()) - (long long)sizeof(AllSmem);
     // the whole matrix with one tile for all rows, or as many rows as fit beside it
     for (int rows = (a.n + kUnitRows - 1) / kUnitRows * kUnitRows; rows >= 2 * kUnitRows && tile == 0; rows -= kUnitRows) {
@@ -471,6 +479,8 @@ bool launch_two_opt_all(const TwoOptArgs& a, int mode, int threads, cudaStream_t
     }
     for (int rows = 4 * kUnitRows; rows >= kUnitRows && tile == 0; rows -= kUnitRows)
       if (2 * (rows + 1) * pitch * 4 + state(rows) <= share) tile = rows;
+    if (tile != 0 || resident == 1) break;
+    --resident;
   }
   if (tile == 0) return false;
   const size_t smem = (size_t)((whole ? a.n : 2 * (tile + 1)) * pitch * 4 + state(tile));
