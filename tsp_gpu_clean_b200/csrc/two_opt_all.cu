@@ -20,7 +20,12 @@
 // first looks in the order of the scan and stops at the first group of rows with an improving
 // pair. Every pair before the last move was not improving, so with symmetric distances the
 // next pass looks at the pairs of earlier rows with the window (when that is the shorter way)
-// and then from the move's row on.
+// and then from the move's row on. On tours far from an optimum the pair is in the first row or
+// two, and copying and evaluating a tile for it is wasted work that costs tours sharing an SM
+// their throughput: while the last pair lay in the first rows of its scan, a warp a row looks at
+// these straight from the matrix before any tile (100 passes of 2400 random tours of 200 cities:
+// 1.2 ms in the general kernel, 1.9 with tiles alone, 0.9). With few tours and a matrix that does
+// not fit, the tiles alone are faster (64 tours of 1000 cities 1.3, 0.59 and 0.79 ms).
 //
 // What bounds it: the chain of a unit (city, row lookups, shuffles, two warp reductions a row)
 // and, for tiles, their copies from L2. Measured through the strategy, before and after: 128
@@ -190,7 +195,8 @@ __device__ __forceinline__ void unit_ahead(RowAt row_at, const int* buf, const i
 
 }  // namespace
 
-template <int MODE>
+// LOOK: first looks at its first rows without a tile.
+template <int MODE, bool LOOK>
 __global__ void __launch_bounds__(kAllThreads) two_opt_all_kernel(const TwoOptArgs A, int tile, int whole, int wide) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ AllSmem S;
@@ -256,6 +262,51 @@ __global__ void __launch_bounds__(kAllThreads) two_opt_all_kernel(const TwoOptAr
   const int rows = n - 2;  // rows i in [0, n - 3]
   const long long exh_total = (long long)(n - 3) + (long long)(n - 3) * (n - 2) / 2;
   long long evals = 0;
+
+  // first: rows [lo, lo + warps) without a tile, a warp per row that leaves at its first
+  // improving pair. Ends with a barrier.
+  auto look = [&](int lo) {
+    const int i = lo + wid;
+    if (i < rows) {
+      const int a = tour[i], b = tour[i + 1], eab = edge[i], lim = n - (i == 0);
+      constexpr int U = 4;  // columns of a lane in flight
+      for (int j0 = i + 2; j0 < lim; j0 += 32 * U) {
+        const unsigned known = *reinterpret_cast<volatile unsigned*>(&S.first);
+        if (__any_sync(FULL, known < (unsigned)i * (unsigned)n)) break;  // an earlier row has a pair
+        int c[U], d[U], dac[U], dbd[U], hit = n;
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int j = j0 + 32 * u + lane;
+          ok[u] = j < lim;
+          c[u] = ok[u] ? tour[j] : a;
+          d[u] = ok[u] ? tour[j + 1 == n ? 0 : j + 1] : b;
+          evals += ok[u];
+        }
+        if (W.whole) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            dac[u] = W.buf[a * W.pitch + c[u]];
+            dbd[u] = W.buf[b * W.pitch + d[u]];
+          }
+        } else {
+          gather_if(A.ds, a, c, ok, dac);
+          gather_if(A.ds, b, d, ok, dbd);
+        }
+#pragma unroll
+        for (int u = U - 1; u >= 0; --u) {
+          const int j = j0 + 32 * u + lane;
+          if (ok[u] && (dac[u] - eab) + (dbd[u] - edge[j]) < 0) hit = j;
+        }
+        hit = __reduce_min_sync(FULL, hit);
+        if (hit < n) {
+          if (lane == 0) atomicMin(&S.first, (unsigned)i * (unsigned)n + (unsigned)hit);
+          break;
+        }
+      }
+    }
+    __syncthreads();
+  };
 
   // Evaluates rows j in [lo, hi]: their pairs with p >= j + 2 when `own`, and the pairs (p, j)
   // of the rows p < p_below. A barrier before (the caller's) and after. first stops after the
@@ -338,6 +389,7 @@ __global__ void __launch_bounds__(kAllThreads) two_opt_all_kernel(const TwoOptAr
   long long passes = 0, moves = 0, pairs_closed = 0;
   int err = TSPB_OK;
   int win_lo = -1, win_hi = -1;  // window of the last move
+  bool near = true;              // first: the last pair found lay in the first rows of its scan
   const long long t_start = clock64();
   while (passes < A.max_iter) {
     if (tid == 0) {
@@ -386,7 +438,17 @@ __global__ void __launch_bounds__(kAllThreads) two_opt_all_kernel(const TwoOptAr
       }
       if (S.first == NO_IDX) {
         __syncthreads();  // S.first is read by all before the scan lowers it
-        evaluate(from, rows - 1, true, 0, true);
+        const int begin = from;
+        if (LOOK && near) {
+          look(from);
+          from += nwarps;
+          const bool found = S.first != NO_IDX;
+          __syncthreads();  // as above
+          if (!found && from < rows) evaluate(from, rows - 1, true, 0, true);
+        } else {
+          evaluate(from, rows - 1, true, 0, true);
+        }
+        near = S.first < (unsigned)(begin + nwarps) * (unsigned)n;
       }
       const unsigned idx = S.first;
       if (tid == 0) {
@@ -451,25 +513,35 @@ __global__ void __launch_bounds__(kAllThreads) two_opt_all_kernel(const TwoOptAr
 // false: the caller takes the general one (distances rebuilt from coordinates, rows too long
 // for tiles of kUnitRows, tours or runs so short that a pass costs less than setting up for it).
 bool launch_two_opt_all(const TwoOptArgs& a, int mode, int threads, cudaStream_t st, int* status) {
+  const bool first = mode == TSPB_MODE_FIRST;
   const int sms = device_attr(cudaDevAttrMultiProcessorCount);
   const int sm_bytes = device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
   if (sms <= 0 || sm_bytes <= 0) return false;
+  const bool many = a.num_tours > sms;  // tours share SMs
   // Below 64 cities a pass is a few hundred cycles and the general kernel's fewer barriers win:
   // 100 tours of 50 cities 0.25 ms there and 0.30 here, of 70 cities 0.46 and 0.38. So they do
   // for the shortest runs: ten passes of 148 tours of 64 cities 0.14 and 0.16 ms, one pass of
-  // 5000 tours of 130 cities 0.25 and 0.32.
+  // 5000 tours of 130 cities 0.25 and 0.32, three first passes of 2400 tours of 300 cities 0.12 and 0.15.
   if (a.ds.dist == nullptr || a.n < 64 || (a.n < 72 && a.max_iter <= 16)) return false;
-  if (a.num_tours > sms && mode == TSPB_MODE_BEST && a.max_iter == 1 && a.n < 300) return false;
+  if (many && (first ? a.max_iter <= 3 : a.max_iter == 1 && a.n < 300)) return false;
   threads = std::min(threads, kAllThreads);
+  // first is a chain of short passes: narrower CTAs, more of them an SM, where there are tours
+  // for it. 30 passes of 1200 tours at 64 / 128 / 256 threads, relative: 64 cities 1.15 / 1 / 0.71,
+  // 200 cities 1.15 / 1 / 0.67, 1000 cities 0.91 / 1 / 0.79; 100 cities 1.10 / 1 / 0.72, but to a
+  // local optimum 0.75 / 1 / 0.64 (at 128 threads the whole matrix of up to 120 cities fits).
+  if (first && a.num_tours >= 2 * sms && a.n < 512) threads = std::min(threads, 128);
+  if (first && (a.n <= 80 ? a.num_tours >= 4 * sms
+                          : a.num_tours >= 8 * sms && a.n < 256 && (a.n >= 128 || a.max_iter <= 64)))
+    threads = std::min(threads, 64);
   const long long pitch = (a.n + 3) & ~3;
   const long long slices = (a.n + kSlice - 1) / kSlice;
   // tour, edges, and best's row keys and two tiles of keys by slice
-  auto state = [&](long long tile) { return (mode == TSPB_MODE_BEST ? 16LL * a.n + 16 * tile * slices : 8LL * a.n) + 16; };
+  auto state = [&](long long tile) { return (first ? 8LL * a.n : 16LL * a.n + 16 * tile * slices) + 16; };
   // CTAs an SM: as many as there are tours for and registers hold. (Shared memory split for more
   // of them than registers hold leaves small tiles: best, ten passes of 5000 tours of 90 cities
   // 1.71 ms that way and 0.81 this, 0.93 in the general kernel.)
-  int resident = std::max(1, std::min((a.num_tours + sms - 1) / sms, kAllThreads / threads));
-  int tile = 0, whole = 0;
+  const int wanted = std::max(1, std::min((a.num_tours + sms - 1) / sms, kAllThreads / threads));
+  int resident = wanted, tile = 0, whole = 0;
   while (true) {
     const long long share = std::min<long long>(sm_bytes / resident - 1024, smem_optin()) - (long long)sizeof(AllSmem);
     // the whole matrix with one tile for all rows, or as many rows as fit beside it
@@ -483,9 +555,15 @@ bool launch_two_opt_all(const TwoOptArgs& a, int mode, int threads, cudaStream_t
     --resident;
   }
   if (tile == 0) return false;
+  // Fewer CTAs than registers hold: a short run of first mode, all of it close to row 0, is
+  // faster in the general kernel, a long one here (2400 tours of 1500 cities, 10 passes: 0.39 ms
+  // there and 0.57 here; 600 of 1000 cities, 100 passes 1.21 and 0.84, 300 on good tours 40 and 9).
+  if (first && resident < wanted && a.max_iter <= 16) return false;
   const size_t smem = (size_t)((whole ? a.n : 2 * (tile + 1)) * pitch * 4 + state(tile));
   const int wide = a.ds.stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.ds.dist) % 16 == 0;
-  auto kern = mode == TSPB_MODE_BEST ? two_opt_all_kernel<TSPB_MODE_BEST> : two_opt_all_kernel<TSPB_MODE_FIRST>;
+  auto kern = !first          ? two_opt_all_kernel<TSPB_MODE_BEST, false>
+              : many || whole ? two_opt_all_kernel<TSPB_MODE_FIRST, true>
+                              : two_opt_all_kernel<TSPB_MODE_FIRST, false>;
   *status = TSPB_ERR_CUDA;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
