@@ -569,8 +569,7 @@ extern "C" int tspb_batch_offspring(const tspb_batch* b, const int32_t* items, i
   if ((long long)num_items * b->P > 0x7fffffffLL) return TSPB_ERR_UNSUPPORTED;
   const size_t smem = offspring_smem_bytes(max_n);
   if (smem > 200 * 1024) return TSPB_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024)
-    TSPB_CUDA_CHECK(cudaFuncSetAttribute(batch_offspring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(batch_offspring_kernel, smem));
   batch_offspring_kernel<<<num_items * b->P, threads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(*b, items, max_n);
   return tspb_launch_status();
 }

@@ -6,10 +6,15 @@
 
 #include "tspb.h"
 
+// A failed call is reported by the status alone: the runtime's last error is taken with it, or
+// the caller's next check of its own would find it.
 #define TSPB_CUDA_CHECK(expr)                                   \
   do {                                                          \
     cudaError_t _e = (expr);                                    \
-    if (_e != cudaSuccess) return TSPB_ERR_CUDA;                \
+    if (_e != cudaSuccess) {                                    \
+      (void)cudaGetLastError();                                 \
+      return TSPB_ERR_CUDA;                                     \
+    }                                                           \
   } while (0)
 
 static inline int tspb_launch_status() {
@@ -17,6 +22,14 @@ static inline int tspb_launch_status() {
 }
 
 namespace tspb {
+
+// Lets `kern` launch with `smem` bytes of dynamic shared memory. A CTA may use 48 KB, its static
+// arrays included, without asking; those of the kernels launched this way take less than 4 KB.
+template <typename Kern>
+static inline cudaError_t allow_smem(Kern kern, size_t smem) {
+  return smem <= 44 * 1024 ? cudaSuccess
+                           : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
 
 constexpr unsigned FULL = 0xffffffffu;
 

@@ -449,7 +449,7 @@ extern "C" int tspb_pmx(const int32_t* parents, int32_t num_routes, int32_t n, c
   if (!parents || !children || (num_routes >= 2 && (!cut_first || !cut_second))) return TSPB_ERR_ARG;
   const size_t smem = (size_t)8 * n + (size_t)((n + 31) / 32) * 4;
   if (smem > 200 * 1024) return TSPB_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(pmx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(pmx_kernel, smem));
   const int threads = n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
   pmx_kernel<<<num_routes, threads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(parents, num_routes, n, cut_first,
                                                                                     cut_second, children, status);
@@ -463,7 +463,7 @@ extern "C" int tspb_ox(const int32_t* parents, int32_t num_routes, int32_t n, co
   if (!parents || !children || (num_routes >= 2 && (!cut_first || !cut_second))) return TSPB_ERR_ARG;
   const size_t smem = (size_t)4 * n + (size_t)3 * ((n + 31) / 32) * 4;
   if (smem > 200 * 1024) return TSPB_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(ox_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(ox_kernel, smem));
   const int threads = n >= 1024 ? 512 : (n >= 256 ? 256 : 128);
   ox_kernel<<<num_routes, threads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(parents, num_routes, n, cut_first,
                                                                                    cut_second, children, status);
@@ -507,8 +507,7 @@ extern "C" int tspb_validate_perm(const int32_t* tours, int32_t num_tours, int32
   if (!bad || (n > 0 && !tours)) return TSPB_ERR_ARG;
   const size_t smem = (size_t)((n + 31) / 32) * 4;
   if (smem > 200 * 1024) return TSPB_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024)
-    TSPB_CUDA_CHECK(cudaFuncSetAttribute(validate_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(validate_perm_kernel, smem));
   validate_perm_kernel<<<num_tours, 256, smem, reinterpret_cast<cudaStream_t>(stream)>>>(tours, n, bad);
   return tspb_launch_status();
 }

@@ -207,8 +207,7 @@ extern "C" int tspb_generation_offspring(const int32_t* pop, const double* fit, 
   if (!dist && !coords) return TSPB_ERR_ARG;
   const size_t smem = offspring_smem_bytes(n);
   if (smem > 200 * 1024) return TSPB_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024)
-    TSPB_CUDA_CHECK(cudaFuncSetAttribute(offspring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(offspring_kernel, smem));
   GenTape tape{tape_tourn, tape_cut_a, tape_cut_b, tape_u, tape_inv_a, tape_inv_b};
   offspring_kernel<<<P, 256, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pop, fit, P, n, kt, tape, gen, stopped, rate,
                                                                              gen_ds(dist, dist_stride, coords), off, off_fit);

@@ -310,8 +310,7 @@ extern "C" int tspb_nn_init_jobs_smem(const tspb_nn_job* jobs, int32_t num_jobs,
   const int stride = (max_n + 7) & ~7;  // 16-byte aligned sub-arrays
   const size_t smem = (size_t)2 * (2 * (size_t)stride + (size_t)((max_k + 7) & ~7));
   if (smem > 200 * 1024) return TSPB_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024)
-    TSPB_CUDA_CHECK(cudaFuncSetAttribute(nn_init_jobs_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(nn_init_jobs_smem_kernel, smem));
   nn_init_jobs_smem_kernel<<<dim3(max_rows, num_jobs), 32, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
       jobs, num_jobs, stride);
   return tspb_launch_status();

@@ -538,7 +538,7 @@ static int launch_or_opt(int32_t* tours, int num, int n, const DistSrc& ds, cons
                          const int32_t* cdist, const uint32_t* packed, int k, int S, long long max_iter,
                          int32_t* status, long long* stats, size_t smem, cudaStream_t st) {
   auto kern = packed ? or_opt_kernel<THREADS, true> : or_opt_kernel<THREADS, false>;
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(kern, smem));
   int per_sm = 0, dev = 0, sms = 0;
   TSPB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem));
   if (per_sm <= 0) return TSPB_ERR_UNSUPPORTED;

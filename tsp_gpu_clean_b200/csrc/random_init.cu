@@ -74,7 +74,7 @@ static int random_init_stage_max(int max_n) { return max_n <= kRandomInitSmemN ?
 
 template <typename K>
 static int set_smem(K kernel, size_t smem) {
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(kernel, smem));
   return TSPB_OK;
 }
 

@@ -444,12 +444,7 @@ extern "C" int tspb_three_opt(int32_t* tours, int32_t num_tours, int32_t n, cons
                   : three_opt_launch<false>(cluster, slots, smem, st, fits, tours, num_tours, n, ds, max_iterations,
                                             workspace, status, s, watchdog_cycles());
   };
-  if (smem > 48 * 1024) {
-    if (smem_m)
-      TSPB_CUDA_CHECK(cudaFuncSetAttribute(three_opt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else
-      TSPB_CUDA_CHECK(cudaFuncSetAttribute(three_opt_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  TSPB_CUDA_CHECK(smem_m ? allow_smem(three_opt_kernel<true>, smem) : allow_smem(three_opt_kernel<false>, smem));
   // the largest cluster for which every tour runs in one wave; tours with fewer units than
   // warps gain nothing from more CTAs
   int cluster = 1;
@@ -463,6 +458,6 @@ extern "C" int tspb_three_opt(int32_t* tours, int32_t num_tours, int32_t n, cons
     }
     (void)cudaGetLastError();
   }
-  if (go(cluster, nullptr) != cudaSuccess) return TSPB_ERR_CUDA;
+  TSPB_CUDA_CHECK(go(cluster, nullptr));
   return tspb_launch_status();
 }

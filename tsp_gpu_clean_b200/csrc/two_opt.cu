@@ -262,7 +262,7 @@ static Layout two_opt_layout(int n, int k, int mode, bool cand) {
 template <int MODE>
 static int launch(const TwoOptArgs& a, int threads, size_t smem, cudaStream_t st) {
   auto kern = a.arrays_in_smem ? two_opt_kernel<MODE, true> : two_opt_kernel<MODE, false>;
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(kern, smem));
   kern<<<a.num_tours, threads, smem, st>>>(a);
   return tspb_launch_status();
 }

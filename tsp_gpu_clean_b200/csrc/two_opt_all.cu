@@ -565,9 +565,10 @@ bool launch_two_opt_all(const TwoOptArgs& a, int mode, int threads, cudaStream_t
               : many || whole ? two_opt_all_kernel<TSPB_MODE_FIRST, true>
                               : two_opt_all_kernel<TSPB_MODE_FIRST, false>;
   *status = TSPB_ERR_CUDA;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (allow_smem(kern, smem) != cudaSuccess) {
+    (void)cudaGetLastError();
     return true;
+  }
   kern<<<a.num_tours, threads, smem, st>>>(a, tile, whole, wide);
   *status = tspb_launch_status();
   return true;

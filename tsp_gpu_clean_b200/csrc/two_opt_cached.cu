@@ -497,7 +497,7 @@ size_t two_opt_cached_tour_bytes(int n, int mode) {
 template <int MODE, int THREADS>
 static int launch_cached(const TwoOptArgs& a, size_t smem, cudaStream_t st) {
   auto kern = a.arrays_in_smem ? two_opt_cached_kernel<MODE, THREADS, true> : two_opt_cached_kernel<MODE, THREADS, false>;
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(kern, smem));
   kern<<<a.num_tours, THREADS, smem, st>>>(a);
   return tspb_launch_status();
 }

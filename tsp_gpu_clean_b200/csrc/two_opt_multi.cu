@@ -359,7 +359,7 @@ int launch_two_opt_multi(const TwoOptArgs& args, int threads, size_t smem, cudaS
       smem = (size_t)arrays + (size_t)cap * 12;
     }
   }
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(kern, smem));
   kern<<<a.num_tours, threads, smem, st>>>(a);
   return tspb_launch_status();
 }

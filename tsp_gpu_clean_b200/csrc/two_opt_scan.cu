@@ -113,7 +113,7 @@ static int launch_scan(const TwoOptArgs& a, size_t smem, cudaStream_t st) {
       kern = a.stats ? two_opt_scan_kernel<MODE, THREADS, U, SCAN_GROUPED, true, true, true>
                      : two_opt_scan_kernel<MODE, THREADS, U, SCAN_GROUPED, true, false, true>;
   }
-  if (smem > 48 * 1024) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TSPB_CUDA_CHECK(allow_smem(kern, smem));
   const int pct = carveout_percent(a.num_tours, smem, ScanMinBlocks<THREADS>::value);
   if (pct > 0) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
   kern<<<a.num_tours, THREADS, smem, st>>>(a);
