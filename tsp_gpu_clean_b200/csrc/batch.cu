@@ -418,7 +418,7 @@ static int batch_two_opt_launch(const tspb_batch& b, const int32_t* items, int n
       int sms = 0, dev = 0;
       TSPB_CUDA_CHECK(cudaGetDevice(&dev));
       TSPB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      const int pct = carveout_for((int)((2 * pairs + sms - 1) / sms), smem);
+      const int pct = carveout_for((int)((2 * pairs + sms - 1) / sms), smem + sizeof(ScanSmem));
       if (pct > 0) TSPB_CUDA_CHECK(cudaFuncSetAttribute(pk, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
       TSPB_CUDA_CHECK(cudaMemsetAsync(queue, 0, sizeof(unsigned), st));
       cfg.gridDim = dim3((unsigned)(2 * pairs));
@@ -441,7 +441,7 @@ static int batch_two_opt_launch(const tspb_batch& b, const int32_t* items, int n
   if (ctas > 0 && ctas < grid) grid = ctas;
   if (grid > units) grid = units;
   const int per_sm_used = (int)((grid + sms - 1) / sms);
-  const int pct = carveout_for(per_sm_used < per_sm ? per_sm_used : per_sm, smem);
+  const int pct = carveout_for(per_sm_used < per_sm ? per_sm_used : per_sm, smem + sizeof(ScanSmem));
   if (pct > 0) TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
   TSPB_CUDA_CHECK(cudaMemsetAsync(queue, 0, sizeof(unsigned), st));
   kern<<<(int)grid, THREADS, smem, st>>>(b, items, num_items, rows, phase, max_iter, max_n, queue, watchdog_cycles());

@@ -544,7 +544,10 @@ static int launch_or_opt(int32_t* tours, int num, int n, const DistSrc& ds, cons
   if (per_sm <= 0) return TSPB_ERR_UNSUPPORTED;
   TSPB_CUDA_CHECK(cudaGetDevice(&dev));
   TSPB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(per_sm, smem)));
+  cudaFuncAttributes own{};  // of its static arrays: they decide whether the last CTA fits
+  TSPB_CUDA_CHECK(cudaFuncGetAttributes(&own, kern));
+  TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       carveout_for(per_sm, smem + own.sharedSizeBytes)));
   const long long grid = (long long)per_sm * sms < num ? (long long)per_sm * sms : num;
   // a row word's low half holds a move's code and a count of entries; beyond it (a segment
   // length times k above 32,768) every pass is a whole scan

@@ -56,6 +56,6 @@ int launch_two_opt_multi(const TwoOptArgs& a, int threads, size_t smem, cudaStre
 int launch_two_opt_scan(const TwoOptArgs& a, int mode, int threads, cudaStream_t st);
 size_t two_opt_scan_tour_bytes(int n, int mode);  // as the workspace sizes state it
 bool two_opt_scan_in_smem(int n, int mode);
-int carveout_for(int ctas_per_sm, size_t smem_per_cta);
+int carveout_for(int ctas_per_sm, size_t cta_bytes);
 
 }  // namespace tspb

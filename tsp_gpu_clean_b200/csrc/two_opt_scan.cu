@@ -49,7 +49,7 @@ bool two_opt_scan_in_smem(int n, int mode) { return scan_tour_state_bytes(n, mod
 static bool scan_counts(const TwoOptArgs& a, int mode) { return mode == TSPB_MODE_FIRST && a.stats != nullptr; }
 
 // Shared-memory carveout (percent of the unified L1/shared array) that holds exactly
-// `ctas_per_sm` CTAs of `smem_per_cta` dynamic bytes; the rest stays L1 for the k-NN
+// `ctas_per_sm` CTAs of `cta_bytes` (static and dynamic) each; the rest stays L1 for the k-NN
 // tables. The default lets the driver take the largest split, which leaves too little L1.
 // An attribute of the current device (queried on every call: a process may drive GPUs of
 // different models, and the query is cheap next to a launch).
@@ -59,10 +59,10 @@ int device_attr(cudaDeviceAttr attr) {
   return v;
 }
 
-int carveout_for(int ctas_per_sm, size_t smem_per_cta) {
+int carveout_for(int ctas_per_sm, size_t cta_bytes) {
   const int smem_sm = device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
   if (smem_sm <= 0 || ctas_per_sm <= 0) return -1;
-  const long long need = (long long)ctas_per_sm * (long long)(smem_per_cta + sizeof(ScanSmem) + 1024);
+  const long long need = (long long)ctas_per_sm * (long long)(cta_bytes + 1024);
   int pct = (int)((need * 100 + smem_sm - 1) / smem_sm);
   return pct < 1 ? 1 : (pct > 100 ? 100 : pct);
 }
@@ -72,7 +72,7 @@ static int carveout_percent(int num_tours, size_t smem_per_cta, int max_ctas_per
   if (sms <= 0) return -1;
   int per_sm = (num_tours + sms - 1) / sms;
   if (per_sm > max_ctas_per_sm) per_sm = max_ctas_per_sm;
-  return carveout_for(per_sm, smem_per_cta);
+  return carveout_for(per_sm, smem_per_cta + sizeof(ScanSmem));
 }
 
 // The grouped layout loads four packed words at once: k % 4 == 0 and a 16-byte aligned table.
