@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 7 : THREADS == 256 ?
       __syncthreads();  // every thread has read s_flag before it is reset
       continue;
     }
-    if (tid == 0) s_wide = cbits == 0;
+    if (tid == 0) s_wide = 0;
     for (int p = tid; p < n; p += THREADS) {
       const int a = st.tour[p];
       st.eout[a] = ds(a, st.at(p + 1));
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 7 : THREADS == 256 ?
     long long cur = 0;  // this thread's share of the valid entries of a pass
     int err = TSPB_OK;
     const long long t0 = clock64();
-    if (cbits != 0 && max_iter > 0) {
+    if (max_iter > 0) {
       bool wide = false;
       for (int q = wgrp; q < n; q += NGROUP) {
         const int a = q + ((tid & 31) / GROUP);
@@ -533,35 +533,245 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 7 : THREADS == 256 ?
   }
 }
 
+// The whole neighbourhood every pass, with 64-bit deltas: for neighbourhoods so small that this
+// takes no longer than keeping the row words does (or_scan_suffices), and for codes too long
+// for a row word. tour, pos, eout and a rebuild buffer in shared memory (16 n bytes); a thread
+// evaluates four consecutive candidates of one (i, L, o), and the move rewrites only the
+// positions between the segment and the insertion point.
+template <int THREADS, bool PACKED>
+__global__ void __launch_bounds__(THREADS) or_scan_kernel(int32_t* __restrict__ tours, int num, int n, DistSrc ds,
+                                                          const int32_t* __restrict__ cand,
+                                                          const int32_t* __restrict__ cdist,
+                                                          const uint32_t* __restrict__ packed, int k, int S,
+                                                          long long max_iter, int32_t* __restrict__ status,
+                                                          long long* __restrict__ stats, long long budget) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ OrMove red[33];
+  __shared__ long long redll[32];
+  __shared__ int s_flag;
+  int* tour = reinterpret_cast<int*>(sm);
+  int* pos = tour + n;
+  int* eout = pos + n;
+  int* tmp = eout + n;
+  const int tid = threadIdx.x;
+  const int chunks = (k + 3) >> 2;
+  const int items = (n - 1) * S * 2 * chunks;  // (i-1, L-1, o) groups x four-candidate chunks
+  for (int t = blockIdx.x; t < num; t += gridDim.x) {
+    int32_t* g = tours + (long long)t * n;
+    if (tid == 0) s_flag = 0;
+    for (int p = tid; p < n; p += THREADS) {
+      tour[p] = g[p];
+      pos[p] = -1;
+    }
+    __syncthreads();
+    for (int p = tid; p < n; p += THREADS) {
+      const int v = tour[p];
+      if ((unsigned)v >= (unsigned)n || atomicExch(&pos[v], p) != -1) s_flag = 1;
+    }
+    __syncthreads();
+    if (s_flag) {
+      if (tid == 0) {
+        status[t] = TSPB_ERR_NOT_PERMUTATION;
+        if (stats)
+          for (int q = 0; q < 3; ++q) stats[(long long)t * 3 + q] = 0;
+      }
+      __syncthreads();  // every thread has read s_flag before it is reset
+      continue;
+    }
+    for (int p = tid; p < n; p += THREADS) {
+      const int a = tour[p];
+      eout[a] = ds(a, tour[p + 1 == n ? 0 : p + 1]);
+    }
+    long long passes = 0, moves = 0, my_eval = 0;
+    int err = TSPB_OK;
+    const long long t0 = clock64();
+    while (passes < max_iter) {
+      __syncthreads();  // the state of the last move (or the setup) is visible
+      if (tid == 0) s_flag = clock64() - t0 > budget;
+      __syncthreads();
+      if (s_flag) {
+        err = TSPB_ERR_BUDGET;
+        break;
+      }
+      OrMove m{0, NO_KEY};
+      for (int it = tid; it < items; it += THREADS) {
+        const int grp = it / chunks, ch = it - grp * chunks;
+        const int o = grp & 1, il = grp >> 1;
+        const int L = il % S + 1, i = il / S + 1;
+        if (i + L - 1 > n - 1 || (o == 1 && L < 2)) continue;
+        const int s0 = tour[i], sl = tour[i + L - 1], p = tour[i - 1], q = tour[i + L == n ? 0 : i + L];
+        const int x = o ? sl : s0, y = o ? s0 : sl;
+        const long long base = (long long)ds(p, q) - eout[p] - eout[sl];
+        const int r0 = ch * 4;
+        int c[4], dxc[4], e[4], dye[4];
+        bool ok[4];
+        if constexpr (PACKED) {  // k % 4 == 0: the four entries exist and are 16-byte aligned
+          const uint4 w = __ldg(reinterpret_cast<const uint4*>(packed + (long long)x * k + r0));
+          const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            ok[u] = true;
+            c[u] = (int)(ws[u] & 0xffffu);
+            dxc[u] = (int)(ws[u] >> 16);
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            ok[u] = r0 + u < k;
+            if (ok[u]) {
+              const long long at = (long long)x * k + r0 + u;
+              c[u] = __ldg(cand + at);
+              dxc[u] = __ldg(cdist + at);
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (!ok[u]) continue;
+          if ((unsigned)c[u] >= (unsigned)n) {
+            ok[u] = false;
+            continue;
+          }
+          const int j = pos[c[u]];
+          ok[u] = j < i - 1 || j > i + L - 1;
+          if (ok[u]) e[u] = tour[j + 1 == n ? 0 : j + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (ok[u]) dye[u] = ds(y, e[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (!ok[u]) continue;
+          ++my_eval;
+          const long long d = base + dxc[u] + dye[u] - eout[c[u]];
+          if (d < 0) {
+            const OrMove v{d, ((((unsigned long long)(i - 1) * S + (L - 1)) * k + (r0 + u)) << 1) | (unsigned)o};
+            if (or_less(v, m)) m = v;
+          }
+        }
+      }
+      ++passes;
+      const OrMove b = block_min_or(m, red);
+      if (b.key == NO_KEY) break;  // a local optimum
+      const int bo = (int)(b.key & 1);
+      const unsigned long long rest = b.key >> 1;
+      const int br = (int)(rest % (unsigned long long)k);
+      const unsigned long long bil = rest / (unsigned long long)k;
+      const int bL = (int)(bil % (unsigned long long)S) + 1, bi = (int)(bil / (unsigned long long)S) + 1;
+      const int bx = bo ? tour[bi + bL - 1] : tour[bi];
+      const int bc = __ldg(cand + (long long)bx * k + br);
+      if ((unsigned)bc >= (unsigned)n) {  // cannot happen for a scanned move; uniform across the CTA
+        err = TSPB_ERR_RANGE;
+        break;
+      }
+      const int bj = pos[bc];
+      if (bj >= bi - 1 && bj <= bi + bL - 1) {
+        err = TSPB_ERR_RANGE;
+        break;
+      }
+      const bool case_a = bj > bi + bL - 1;
+      const int lo = case_a ? bi : bj + 1, hi = case_a ? bj : bi + bL - 1;
+      for (int np = lo + tid; np <= hi; np += THREADS) {
+        int v;
+        if (case_a) {
+          if (np <= bj - bL) {
+            v = tour[np + bL];
+          } else {
+            const int mm = np - (bj - bL + 1);
+            v = bo ? tour[bi + bL - 1 - mm] : tour[bi + mm];
+          }
+        } else {
+          if (np <= bj + bL) {
+            const int mm = np - (bj + 1);
+            v = bo ? tour[bi + bL - 1 - mm] : tour[bi + mm];
+          } else {
+            v = tour[np - bL];
+          }
+        }
+        tmp[np] = v;
+      }
+      __syncthreads();
+      for (int np = lo + tid; np <= hi; np += THREADS) {
+        const int v = tmp[np];
+        tour[np] = v;
+        pos[v] = np;
+      }
+      __syncthreads();
+      for (int np = lo - 1 + tid; np <= hi; np += THREADS) {
+        const int a = tour[np];
+        eout[a] = ds(a, tour[np + 1 == n ? 0 : np + 1]);
+      }
+      ++moves;
+    }
+    __syncthreads();
+    for (int p = tid; p < n; p += THREADS) g[p] = tour[p];
+    const long long ev = block_sum(my_eval, redll);
+    if (tid == 0) {
+      status[t] = err;
+      if (stats) {
+        stats[(long long)t * 3 + 0] = passes;
+        stats[(long long)t * 3 + 1] = moves;
+        stats[(long long)t * 3 + 2] = ev;
+      }
+    }
+    __syncthreads();  // tour, s_flag and redll are reused by the next tour
+  }
+}
+
+// CTAs of a launch: all that run at once, one per tour at most; 0: a CTA does not fit, -1: a
+// runtime error.
+template <typename Kern>
+static int or_grid(Kern kern, int threads, int num, size_t smem, bool carveout) {
+  int per_sm = 0;
+  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
+  if (sms <= 0 || allow_smem(kern, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return -1;
+  }
+  if (per_sm > 0 && carveout) {
+    cudaFuncAttributes own{};  // of its static arrays: they decide whether the last CTA fits
+    if (cudaFuncGetAttributes(&own, kern) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             carveout_for(per_sm, smem + own.sharedSizeBytes)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return -1;
+    }
+  }
+  return (int)((long long)per_sm * sms < num ? (long long)per_sm * sms : num);
+}
+
+// Whether evaluating everything each pass is the faster way. A scan costs about four units an
+// item of up to four candidates and one a candidate; keeping rows costs a pass of fixed phases
+// that grow with the segment length, and, where tours share SMs, of phases that grow with n.
+// 50 passes, scan and rows, in ms: segments of 1, one tour of 50 cities, k = 8 0.28 and 0.35, of
+// 100 cities 0.42 and 0.36; 2000 tours of 1000 cities, k = 1 2.6 and 4.8. Segments up to 3, k = 3,
+// 1000 tours of 50 cities 0.40 and 0.47, of 100 0.82 and 0.60.
+static bool or_scan_suffices(int num, int n, int k, int S) {
+  const long long cost = (long long)n * (2 * S - 1) * (4 * ((k + 3) / 4) + k) / 8;
+  return cost < 60 + 85 * S ||
+         (S == 1 && k <= 3 && n < 2000 && num > 3 * device_attr(cudaDevAttrMultiProcessorCount));
+}
+
 template <int THREADS>
 static int launch_or_opt(int32_t* tours, int num, int n, const DistSrc& ds, const int32_t* cand,
-                         const int32_t* cdist, const uint32_t* packed, int k, int S, long long max_iter,
+                         const int32_t* cdist, const uint32_t* packed, int k, int S, int cbits, long long max_iter,
                          int32_t* status, long long* stats, size_t smem, cudaStream_t st) {
+  if (cbits == 0) {  // whole scans
+    auto scan = packed ? or_scan_kernel<THREADS, true> : or_scan_kernel<THREADS, false>;
+    const int grid = or_grid(scan, THREADS, num, smem, false);
+    if (grid <= 0) return grid < 0 ? TSPB_ERR_CUDA : TSPB_ERR_UNSUPPORTED;
+    scan<<<grid, THREADS, smem, st>>>(tours, num, n, ds, cand, cdist, packed, k, S, max_iter, status, stats,
+                                      watchdog_cycles());
+    return tspb_launch_status();
+  }
   auto kern = packed ? or_opt_kernel<THREADS, true> : or_opt_kernel<THREADS, false>;
-  TSPB_CUDA_CHECK(allow_smem(kern, smem));
-  int per_sm = 0, dev = 0, sms = 0;
-  TSPB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem));
-  if (per_sm <= 0) return TSPB_ERR_UNSUPPORTED;
-  TSPB_CUDA_CHECK(cudaGetDevice(&dev));
-  TSPB_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  cudaFuncAttributes own{};  // of its static arrays: they decide whether the last CTA fits
-  TSPB_CUDA_CHECK(cudaFuncGetAttributes(&own, kern));
-  TSPB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       carveout_for(per_sm, smem + own.sharedSizeBytes)));
-  const long long grid = (long long)per_sm * sms < num ? (long long)per_sm * sms : num;
-  // a row word's low half holds a move's code and a count of entries; beyond it (a segment
-  // length times k above 32,768) every pass is a whole scan
-  auto bits = [](unsigned v) {
-    int b = 0;
-    while (v >> b) ++b;
-    return b;
-  };
-  int cbits = bits((unsigned)(2 * S - 1) * (unsigned)k);
-  if (cbits + bits(2u * (unsigned)S * (unsigned)k - 1) > 32) cbits = 0;
+  const int grid = or_grid(kern, THREADS, num, smem, true);
+  if (grid <= 0) return grid < 0 ? TSPB_ERR_CUDA : TSPB_ERR_UNSUPPORTED;
   const void* table = packed ? static_cast<const void*>(packed) : cand;
   const int vec = reinterpret_cast<uintptr_t>(table) % 16 == 0;
-  kern<<<(int)grid, THREADS, smem, st>>>(tours, num, n, ds, cand, cdist, packed, k, S, cbits, vec, max_iter, status,
-                                         stats, watchdog_cycles());
+  kern<<<grid, THREADS, smem, st>>>(tours, num, n, ds, cand, cdist, packed, k, S, cbits, vec, max_iter, status, stats,
+                                    watchdog_cycles());
   return tspb_launch_status();
 }
 
@@ -596,27 +806,37 @@ extern "C" int tspb_or_opt(int32_t* tours, int32_t num_tours, int32_t n, const i
   // the packed words serve only whole, aligned groups of four
   const uint32_t* pk =
       cand_packed && k % 4 == 0 && reinterpret_cast<uintptr_t>(cand_packed) % 16 == 0 ? cand_packed : nullptr;
+  // a row word's low half holds a move's code and a count of entries
+  auto bits = [](unsigned v) {
+    int b = 0;
+    while (v >> b) ++b;
+    return b;
+  };
+  int cbits = bits((unsigned)(2 * max_segment - 1) * (unsigned)k);
+  if (cbits + bits(2u * (unsigned)max_segment * (unsigned)k - 1) > 32) cbits = 0;
+  const bool small = or_scan_suffices(num_tours, n, k, max_segment);
+  if (small) cbits = 0;
   // Where tours leave SMs or warps idle a pass is a chain of latencies, and a wider CTA
   // shortens it. 50 passes, k = 20: one tour of 1000 cities 1.01 / 0.66 / 0.58 ms at 128 /
   // 256 / 512 threads, 300 of them 1.27 / 1.09 / 1.73, 1024 of them 2.34 / 2.73 / 4.07; 400
   // of 200 cities 0.76 / 0.98 / 1.33; 64 of 300 (k = 10) 0.40 / 0.35 / 0.36.
   const int sms = device_attr(cudaDevAttrMultiProcessorCount);
   const bool large = (long long)n * k >= 16384;
-  if (num_tours <= sms) {
+  if (!small && num_tours <= sms) {
     const int w = large ? 512 : 256;
     threads = threads > w ? threads : w;
-  } else if (num_tours <= 3 * sms && large && threads < 256) {
+  } else if (!small && num_tours <= 3 * sms && large && threads < 256) {
     threads = 256;
   }
   switch (threads) {
     case 128:
-      return launch_or_opt<128>(tours, num_tours, n, ds, cand, cand_dist, pk, k, max_segment, max_iterations, status, s,
-                                smem, st);
+      return launch_or_opt<128>(tours, num_tours, n, ds, cand, cand_dist, pk, k, max_segment, cbits, max_iterations, status,
+                                s, smem, st);
     case 512:
-      return launch_or_opt<512>(tours, num_tours, n, ds, cand, cand_dist, pk, k, max_segment, max_iterations, status, s,
-                                smem, st);
+      return launch_or_opt<512>(tours, num_tours, n, ds, cand, cand_dist, pk, k, max_segment, cbits, max_iterations, status,
+                                s, smem, st);
     default:
-      return launch_or_opt<256>(tours, num_tours, n, ds, cand, cand_dist, pk, k, max_segment, max_iterations, status, s,
-                                smem, st);
+      return launch_or_opt<256>(tours, num_tours, n, ds, cand, cand_dist, pk, k, max_segment, cbits, max_iterations, status,
+                                s, smem, st);
   }
 }
