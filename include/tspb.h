@@ -529,7 +529,7 @@ typedef struct tspb_batch {
   double* fit[2];           /* [I][P] */
   int32_t* off;             /* offspring rows (pop layout) */
   double* off_fit;          /* [I][P] */
-  int32_t* order;           /* [I][P] survival scratch */
+  int32_t* order;           /* [I][P] the survivors' sources: a row of the population, or P + one of the offspring */
   const int32_t* tape_tourn; /* [I][G][P][kt] */
   const int32_t* tape_cut_a; /* [I][G][P/2] */
   const int32_t* tape_cut_b; /* [I][G][P/2] */
@@ -562,6 +562,8 @@ int tspb_batch_offspring(const tspb_batch* b, const int32_t* items, int32_t num_
 /* Survival of every RUN instance and the elite-edge tie rule (RUN -> PAUSED); replaces
  * _select_survivors_assessed (genetic_algorithm.py:618-706) for every run. */
 int tspb_batch_survival(const tspb_batch* b, void* stream);
+/* Kernels that tspb_batch_survival launches for a batch of this size. */
+int tspb_batch_survival_launches(int32_t num_instances, int32_t population);
 #define TSPB_BATCH_COORDS 1  /* every item has dist == NULL: distances rebuilt from coordinates */
 #define TSPB_BATCH_GROUPED 2 /* every item's k is a multiple of 4 and its packed table 16-byte aligned */
 /* with GROUPED: every item has rev_off/rev_idx. Best mode keeps the minimum improving key

@@ -369,10 +369,10 @@ class FusedBatchSolver:
     native.check("tspb_batch_track", lib.tspb_batch_track(st, U, sh))
     self.kernel_launches += 1
 
-  @staticmethod
-  def _survival_launches() -> int:
-    """Kernels of tspb_batch_survival: rank, elite-edge tie check and survivor copy in one."""
-    return 1
+  def _survival_launches(self) -> int:
+    """Kernels of tspb_batch_survival: rank, elite-edge tie check and survivor copy in one, or
+    the rank and the copy apart where the batch is large."""
+    return int(native.load_library().tspb_batch_survival_launches(self.I, self.P))
 
   def _launches_per_replay(self, resume: bool = False) -> int:
     nb = len(self.buckets)

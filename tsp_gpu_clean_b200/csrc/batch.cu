@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(256) batch_offspring_kernel(const tspb_batch B
 // Counting costs 2P comparisons a CTA over values that stay in L2, with no order between
 // CTAs, where a sort of the 2P pairs is a chain of barriers on one SM and a launch of its
 // own: P = 512, n = 1000 4.0 us against 8.4 for the sort and 3.5 for the copies; 128 runs of
-// 64 rows (1,075 cities on average) 31.7 against 4.9 + 27.9, bound by the copies.
+// 64 rows (1,075 cities on average) 31.7 against 4.9 + 27.9, bound by the copies. Its work grows
+// with the runs times P squared: larger batches are sorted (survival_counts).
 constexpr int SURVIVAL_THREADS = 128;
 __global__ void __launch_bounds__(SURVIVAL_THREADS) batch_survival_kernel(const tspb_batch B) {
   const int P = B.P, count = 2 * P;
@@ -203,6 +204,201 @@ __global__ void __launch_bounds__(SURVIVAL_THREADS) batch_survival_kernel(const 
       if (tie && !clean) B.ctl[4 * i + 1] = TSPB_BATCH_PAUSED;
     }
   }
+}
+
+// The elite-edge tie of generation g, settled by the whole CTA right after the survival
+// sort: key[r], idx[r] (shared memory, r < P) are the survivors' fitness and source index
+// (< P: the population, else the offspring). Positions elite-1 and elite with equal fitness
+// let NumPy's unstable argsort choose the elites. The run goes on when every survivor of
+// that fitness is converged (any choice refines only rows that do not change), else it
+// pauses for the host's argsort. The survivors are gathered in the same generation whether
+// the run pauses or not (the gather serves RUN and PAUSED runs).
+__device__ void survival_tie(const tspb_batch& B, int i, int g, int parity, const double* key, const int* idx) {
+  const int P = B.P, e = B.elite;
+  if (e <= 0 || e >= P) return;  // uniform: no edge
+  const double fe = key[e - 1];
+  const bool tie = key[e] == fe;
+  bool ok = true;
+  if (tie) {
+    if (!B.clean[0]) {
+      ok = false;
+    } else {
+      const uint8_t* ca = clean_buf(B, parity) + (long long)i * P;
+      const uint8_t* cb = B.off_clean + (long long)i * P;
+      for (int r = threadIdx.x; r < P; r += blockDim.x)
+        if (key[r] == fe) ok = ok && (idx[r] < P ? ca[idx[r]] : cb[idx[r] - P]) != 0;
+    }
+  }
+  const int settled = __syncthreads_and(ok ? 1 : 0);
+  if (threadIdx.x == 0) {
+    B.ties[(long long)i * B.G + g] = tie ? 1 : 0;
+    if (tie && !settled) B.ctl[4 * i + 1] = TSPB_BATCH_PAUSED;
+  }
+}
+
+// CTA per instance: the stable order of the 2P combined fitness values (old population
+// first), i.e. (fitness, index) ascending, as the reference's lexsort keeps it; the first P
+// indices go to order[], then the elite-edge tie. A bitonic sort of (fitness, index) pairs
+// in shared memory, padded with +inf to the next power of two n2.
+__global__ void batch_survival_rank_kernel(const tspb_batch B, int n2) {
+  extern __shared__ __align__(16) unsigned char rank_sm[];
+  double* key = reinterpret_cast<double*>(rank_sm);
+  int* idx = reinterpret_cast<int*>(key + n2);
+  const int i = blockIdx.x, P = B.P;
+  const int* c = B.ctl + 4 * i;
+  if (c[1] != TSPB_BATCH_RUN) return;
+  const int parity = c[0] & 1;
+  const double* fa = fit_buf(B, parity) + (long long)i * P;
+  const double* fb = B.off_fit + (long long)i * P;
+  const int count = 2 * P;
+  for (int j = threadIdx.x; j < n2; j += blockDim.x) {
+    key[j] = j < P ? fa[j] : (j < count ? fb[j - P] : __longlong_as_double(0x7ff0000000000000LL));
+    idx[j] = j;
+  }
+  __syncthreads();
+  for (int kk = 2; kk <= n2; kk <<= 1) {
+    for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+      for (int t = threadIdx.x; t < n2; t += blockDim.x) {
+        const int u = t ^ jj;
+        if (u > t) {
+          const double kt = key[t], ku = key[u];
+          const int it = idx[t], iu = idx[u];
+          const bool t_after_u = kt > ku || (kt == ku && it > iu);
+          if (t_after_u == ((t & kk) == 0)) {
+            key[t] = ku;
+            key[u] = kt;
+            idx[t] = iu;
+            idx[u] = it;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int r = threadIdx.x; r < P; r += blockDim.x) B.order[(long long)i * P + r] = idx[r];
+  survival_tie(B, i, c[0], parity, key, idx);
+}
+
+// The same order with n2 / 2 threads (64 <= n2 <= 2048): thread t holds positions t and
+// t + n2/2 in registers. A compare-exchange at distance j pairs positions e and e ^ j: for
+// j < 32 the partner sits in the same warp (lane ^ j, same slot), for j = n2/2 it is the
+// thread's other slot, otherwise the pair meets in shared memory. Each position keeps the
+// smaller (fitness, index) when it is the lower one of an ascending pair ((e & k) == 0) or
+// the higher one of a descending pair, as in the shared-memory sort above.
+__device__ __forceinline__ bool rank_after(double ka, int ia, double kb, int ib) {
+  return ka > kb || (ka == kb && ia > ib);
+}
+
+__device__ __forceinline__ void rank_keep(double& k, int& id, double pk, int pid, int e, int p, int kk) {
+  const bool asc = (e & kk) == 0;
+  const bool want_small = (e < p) == asc;
+  if (rank_after(k, id, pk, pid) == want_small) {  // the partner is the one this position keeps
+    k = pk;
+    id = pid;
+  }
+}
+
+__global__ void batch_survival_rank_reg_kernel(const tspb_batch B, int n2) {
+  extern __shared__ __align__(16) unsigned char rank_sm[];
+  double* skey = reinterpret_cast<double*>(rank_sm);
+  int* sidx = reinterpret_cast<int*>(skey + n2);
+  const int i = blockIdx.x, P = B.P;
+  const int* c = B.ctl + 4 * i;
+  if (c[1] != TSPB_BATCH_RUN) return;  // uniform per CTA
+  const int parity = c[0] & 1;
+  const double* fa = fit_buf(B, parity) + (long long)i * P;
+  const double* fb = B.off_fit + (long long)i * P;
+  const int half = n2 >> 1, t = threadIdx.x, count = 2 * P;
+  const double inf = __longlong_as_double(0x7ff0000000000000LL);
+  auto load = [&](int e) { return e < P ? fa[e] : (e < count ? fb[e - P] : inf); };
+  const int e0 = t, e1 = t + half;
+  double k0 = load(e0), k1 = load(e1);
+  int i0 = e0, i1 = e1;
+  for (int kk = 2; kk <= n2; kk <<= 1) {
+    for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+      if (jj == half) {  // e1 = e0 ^ half: both in this thread (kk == n2, ascending)
+        if (rank_after(k0, i0, k1, i1)) {
+          const double tk = k0;
+          const int ti = i0;
+          k0 = k1;
+          i0 = i1;
+          k1 = tk;
+          i1 = ti;
+        }
+      } else if (jj < 32) {
+        const double p0 = __shfl_xor_sync(FULL, k0, jj), p1 = __shfl_xor_sync(FULL, k1, jj);
+        const int q0 = __shfl_xor_sync(FULL, i0, jj), q1 = __shfl_xor_sync(FULL, i1, jj);
+        rank_keep(k0, i0, p0, q0, e0, e0 ^ jj, kk);
+        rank_keep(k1, i1, p1, q1, e1, e1 ^ jj, kk);
+      } else {
+        skey[e0] = k0;
+        sidx[e0] = i0;
+        skey[e1] = k1;
+        sidx[e1] = i1;
+        __syncthreads();
+        const double p0 = skey[e0 ^ jj], p1 = skey[e1 ^ jj];
+        const int q0 = sidx[e0 ^ jj], q1 = sidx[e1 ^ jj];
+        __syncthreads();  // every partner read before the next stage writes
+        rank_keep(k0, i0, p0, q0, e0, e0 ^ jj, kk);
+        rank_keep(k1, i1, p1, q1, e1, e1 ^ jj, kk);
+      }
+    }
+  }
+  if (e0 < P) {  // half >= P: slot 1 is never a survivor
+    B.order[(long long)i * P + e0] = i0;
+    skey[e0] = k0;  // the sorted survivors for the tie check (every earlier read is behind a barrier)
+    sidx[e0] = i0;
+  }
+  __syncthreads();
+  survival_tie(B, i, c[0], parity, skey, sidx);
+}
+
+// CTA per (instance, survivor): new_pop[r] = combined[order[r]] with its fitness and
+// converged bit. A run the rank kernel just paused is gathered too (the host's argsort
+// reads the survivors); a run still waiting for the host is gathered again in later
+// replays from the same unchanged order, population and offspring, which rewrites the
+// same rows.
+__global__ void __launch_bounds__(SURVIVAL_THREADS) batch_survival_gather_kernel(const tspb_batch B) {
+  const int P = B.P;
+  const int i = blockIdx.x / P, r = blockIdx.x - i * P;
+  const int* c = B.ctl + 4 * i;
+  if (c[1] != TSPB_BATCH_RUN && c[1] != TSPB_BATCH_PAUSED) return;
+  const int g = c[0], parity = g & 1;
+  const tspb_batch_instance I = B.inst[i];
+  const int n = I.n;
+  const int32_t* order = B.order + (long long)i * P;
+  const double* fit = fit_buf(B, parity) + (long long)i * P;
+  const double* off_fit = B.off_fit + (long long)i * P;
+  const int o = order[r];
+  const int32_t* src = o < P ? pop_buf(B, parity) + I.pop_offset + (long long)o * n
+                             : B.off + I.pop_offset + (long long)(o - P) * n;
+  int32_t* dst = pop_buf(B, parity ^ 1) + I.pop_offset + (long long)r * n;
+  if ((n & 3) == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+    const int4* s4 = reinterpret_cast<const int4*>(src);
+    int4* d4 = reinterpret_cast<int4*>(dst);
+    for (int t = threadIdx.x; t < (n >> 2); t += blockDim.x) d4[t] = s4[t];
+  } else {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) dst[t] = src[t];
+  }
+  if (threadIdx.x == 0) {
+    const double f = o < P ? fit[o] : off_fit[o - P];
+    fit_buf(B, parity ^ 1)[(long long)i * P + r] = f;
+    if (B.clean[0]) {
+      const uint8_t* cs = clean_buf(B, parity) + (long long)i * P;
+      clean_buf(B, parity ^ 1)[(long long)i * P + r] = o < P ? cs[o] : B.off_clean[(long long)i * P + o - P];
+    }
+  }
+}
+
+// Whether survivors are ranked by counting (one launch) instead of by a sort per instance (two).
+// Measured: a member counts for 0.85 ns and 1.7 ns per thousand rows more than its copy alone takes,
+// an instance's sort takes 10 us and 12.5 more per thousand rows up to 1024 of them, P^2 / 52,000 us
+// above (registers do not hold the pairs). 16 runs of 512 rows 21 us either way; 64 of 1024 196
+// counted and 70 sorted, 4 of 3072 89 and 188, 128 of 64 15 and 17.
+static bool survival_counts(int instances, int P) {
+  const long long members = (long long)instances * P;
+  const long long sort_ps = P <= 1024 ? 10000000LL + 12500LL * P : 19LL * P * P;
+  return 2 * members <= 0x7fffffffLL && members * (850 + 17LL * P / 10) < sort_ps;
 }
 
 // Persistent 2-opt over the (item, row) units of one phase. COORDS: the bucket's
@@ -577,10 +773,28 @@ extern "C" int tspb_batch_offspring(const tspb_batch* b, const int32_t* items, i
 extern "C" int tspb_batch_survival(const tspb_batch* b, void* stream) {
   if (!batch_ok(b) || !tape_ok(b)) return TSPB_ERR_ARG;
   if (b->num_instances == 0 || b->G == 0) return TSPB_OK;
-  if (2LL * b->num_instances * b->P > 0x7fffffffLL || b->P > 3072) return TSPB_ERR_UNSUPPORTED;
+  if ((long long)b->num_instances * b->P > 0x7fffffffLL || b->P > 3072) return TSPB_ERR_UNSUPPORTED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  batch_survival_kernel<<<2 * b->num_instances * b->P, SURVIVAL_THREADS, 0, st>>>(*b);
+  if (survival_counts(b->num_instances, b->P)) {
+    batch_survival_kernel<<<2 * b->num_instances * b->P, SURVIVAL_THREADS, 0, st>>>(*b);
+    return tspb_launch_status();
+  }
+  int n2 = 1;
+  while (n2 < 2 * b->P) n2 <<= 1;
+  const size_t rank_smem = (size_t)12 * n2;
+  if (n2 >= 64 && n2 <= 2048) {  // n2 / 2 threads, pairs in registers
+    batch_survival_rank_reg_kernel<<<b->num_instances, n2 / 2, rank_smem, st>>>(*b, n2);
+  } else {
+    const int rank_threads = n2 >= 1024 ? 512 : (n2 / 2 > 32 ? n2 / 2 : 32);
+    TSPB_CUDA_CHECK(allow_smem(batch_survival_rank_kernel, rank_smem));
+    batch_survival_rank_kernel<<<b->num_instances, rank_threads, rank_smem, st>>>(*b, n2);
+  }
+  batch_survival_gather_kernel<<<b->num_instances * b->P, SURVIVAL_THREADS, 0, st>>>(*b);
   return tspb_launch_status();
+}
+
+extern "C" int tspb_batch_survival_launches(int32_t num_instances, int32_t population) {
+  return survival_counts(num_instances, population) ? 1 : 2;
 }
 
 extern "C" int tspb_batch_two_opt_occupancy(int32_t max_n, int32_t mode, int32_t threads, int32_t flags) {
