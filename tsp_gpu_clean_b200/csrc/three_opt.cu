@@ -164,7 +164,7 @@ __device__ __forceinline__ MoveKey scan_pass(const int* M, const int* edge, int 
   constexpr int JB = kUnitJ<D>;
   int turn = 0;
   for (int k_lo = (n - 1) & ~31; k_lo >= 0; k_lo -= 32) {
-    for (int jb = 0; jb <= k_lo + 30 && jb < n - 2; jb += JB) {
+    for (int jb = 0; jb <= k_lo + 30 && jb <= n - 2; jb += JB) {
       const int k_hi = k_lo + 31 < n - 1 ? k_lo + 31 : n - 1;
       const int j_end = jb + JB - 1 < k_hi - 1 ? jb + JB - 1 : k_hi - 1;
       if (j_end < 1 || j_end < jb) continue;
