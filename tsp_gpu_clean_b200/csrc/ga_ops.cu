@@ -273,6 +273,32 @@ __global__ void __launch_bounds__(INVERSION_THREADS) inversion_kernel(int32_t* _
   }
 }
 
+// The same with a warp per route: most routes leave at once, and a CTA for each costs more to
+// start than a short reversal takes (inversion_per_cta).
+__global__ void __launch_bounds__(256) inversion_warp_kernel(int32_t* __restrict__ routes, int num_routes, int n,
+                                                             const double* __restrict__ u, double rate,
+                                                             const int32_t* __restrict__ pos1,
+                                                             const int32_t* __restrict__ pos2) {
+  const int r = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (r >= num_routes) return;
+  if (!(__ldg(u + r) < rate)) return;
+  const int a = __ldg(pos1 + r), b = __ldg(pos2 + r);
+  const int lo = a < b ? a : b, hi = a < b ? b : a;
+  if (lo < 0 || hi >= n) return;
+  int32_t* t = routes + (long long)r * n;
+  const int half = (hi - lo + 1) >> 1;
+  for (int q = threadIdx.x & 31; q < half; q += 32) {
+    const int x = t[lo + q], y = t[hi - q];
+    t[lo + q] = y;
+    t[hi - q] = x;
+  }
+}
+
+// CTAs pay where the reversal is the longer part and the routes are few: 4096 routes of 1000 cities
+// 13.4 us (16.2 with warps), 2000 of 5000 21 (35), 16,384 of 1000 20 either way; with warps 65,536
+// of 50 take 13 us (42 with CTAs), a million of 20 73 (524).
+static bool inversion_per_cta(int num_routes, int n) { return n >= 512 && num_routes <= 16384; }
+
 // Thread per element: rank by (value, index); ranks below `keep` scatter the index
 // (a stable ascending sort, np.lexsort of genetic_algorithm.py:682-689).
 __global__ void stable_rank_kernel(const double* __restrict__ f, int count, int keep, int32_t* __restrict__ order) {
@@ -486,8 +512,13 @@ extern "C" int tspb_inversion(int32_t* routes, int32_t num_routes, int32_t n, co
   if (num_routes < 0 || n < 0) return TSPB_ERR_ARG;
   if (num_routes == 0 || n == 0) return TSPB_OK;
   if (!routes || !u || !pos1 || !pos2) return TSPB_ERR_ARG;
-  inversion_kernel<<<num_routes, INVERSION_THREADS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(routes, num_routes, n, u,
-                                                                                               rate, pos1, pos2);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (inversion_per_cta(num_routes, n)) {
+    inversion_kernel<<<num_routes, INVERSION_THREADS, 0, st>>>(routes, num_routes, n, u, rate, pos1, pos2);
+  } else {
+    const int blocks = (int)(((long long)num_routes * 32 + 255) / 256);
+    inversion_warp_kernel<<<blocks, 256, 0, st>>>(routes, num_routes, n, u, rate, pos1, pos2);
+  }
   return tspb_launch_status();
 }
 
