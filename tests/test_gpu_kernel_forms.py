@@ -39,3 +39,36 @@ def test_inversion(routes, n):
   d = [torch.from_numpy(x).cuda() for x in (tours, u, a, b)]
   native.call("tspb_inversion", ptr(d[0]), routes, n, ptr(d[1]), 0.5, ptr(d[2]), ptr(d[3]), stream_handle())
   assert np.array_equal(d[0].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n,pool_k", [(60, 10), (60, 11), (256, 128), (257, 128), (993, 33)])
+@pytest.mark.parametrize("matrix", [True, False])
+def test_edge_features(n, pool_k, matrix):
+  torch, native, ptr, stream_handle = _gpu()
+  rng = np.random.default_rng(n)
+  coords = rng.uniform(0.0, 1000.0, (n, 2))
+  D = odist.euc2d_matrix(coords)
+  pool = odist.candidate_list(pool_k, distances=D)
+  pos = rng.permutation(n).astype(np.int32)
+  f32 = np.float32
+  rank = np.full((n, n), pool_k)  # rank[v, u]: slot of u in v's pool
+  np.put_along_axis(rank, pool, np.broadcast_to(np.arange(pool_k), pool.shape), axis=1)
+  U = np.arange(n)[:, None]
+  su = np.maximum(D[np.arange(n), pool[:, -1]], 1).astype(f32)[:, None]
+  x = np.zeros((n, pool_k, 16), dtype=f32)
+  x[..., 0] = D[U, pool].astype(f32) / su
+  x[..., 1] = np.arange(pool_k, dtype=f32) / f32(pool_k)
+  x[..., 2] = rank[pool, U].astype(f32) / f32(pool_k)
+  x[..., 3] = (coords[pool, 0] - coords[U, 0]).astype(f32) / su
+  x[..., 4] = (coords[pool, 1] - coords[U, 1]).astype(f32) / su
+  gap = np.abs(pos[U] - pos[pool])
+  y = ((gap == 1) | (gap == n - 1)).astype(f32)
+  want = torch.from_numpy(x).to(torch.bfloat16).view(torch.int16)
+  c, p, t = torch.from_numpy(coords).cuda(), torch.from_numpy(pool).cuda(), torch.from_numpy(pos).cuda()
+  d = torch.from_numpy(D).cuda() if matrix else None
+  got = torch.empty((n, pool_k, 16), dtype=torch.int16, device="cuda")
+  lab = torch.empty((n, pool_k), dtype=torch.float32, device="cuda")
+  native.call("tspb_edge_features", ptr(c), n, ptr(p), pool_k, ptr(d), n if matrix else 0, ptr(t), ptr(got), ptr(lab),
+              stream_handle())
+  assert torch.equal(got.cpu(), want)
+  assert np.array_equal(lab.cpu().numpy(), y)

@@ -325,7 +325,34 @@ __global__ void adam_kernel(float* __restrict__ P, float* __restrict__ grad, flo
 //   d(u,v)/s_u, s/P, rank of u in pool[v] / P (1 when absent), (x_v-x_u)/s_u, (y_v-y_u)/s_u
 // with s_u = max(d(u, pool[u][P-1]), 1). Labels (optional): 1 when v follows or precedes u
 // in `tour_pos` order (tour_pos[node] = position), else 0.
-//
+__device__ __forceinline__ void edge_row(const double2* __restrict__ coords, int n, const DistSrc& ds,
+                                         const int32_t* __restrict__ tour_pos, int u, int s, int v, int PK, float su,
+                                         int rvu, uint32_t* __restrict__ X32, float* __restrict__ y) {
+  float f[MLP_F] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  float label = 0.f;
+  if ((unsigned)v < (unsigned)n) {
+    const double2 pu = coords[u], pv = coords[v];
+    f[0] = (float)ds(u, v) / su;
+    f[1] = (float)s / (float)PK;
+    f[2] = (float)rvu / (float)PK;
+    f[3] = (float)(pv.x - pu.x) / su;
+    f[4] = (float)(pv.y - pu.y) / su;
+    if (tour_pos) {
+      const int pu_ = tour_pos[u], pv_ = tour_pos[v];
+      const int dpos = pu_ > pv_ ? pu_ - pv_ : pv_ - pu_;
+      label = (dpos == 1 || dpos == n - 1) ? 1.f : 0.f;
+    }
+  }
+  const long long e = (long long)u * PK + s;
+  uint32_t* row = X32 + e * 8;
+  row[0] = pack_bf16(f[0], f[1]);
+  row[1] = pack_bf16(f[2], f[3]);
+  row[2] = pack_bf16(f[4], 0.f);
+#pragma unroll
+  for (int q = 3; q < 8; ++q) row[q] = 0u;
+  if (y) y[e] = label;
+}
+
 // A warp per node u. The rank of u in each neighbour's pool is found with the lanes over that
 // pool (one coalesced read and a ballot per neighbour), where a thread per edge walked it
 // alone through up to PK scattered reads (n = 10,000, PK = 30: 23.9 -> 19.2 us).
@@ -339,7 +366,6 @@ __global__ void __launch_bounds__(256) edge_features_kernel(const double2* __res
   const int32_t* mine = pool + (long long)u * PK;
   const int far = __ldg(mine + PK - 1);
   const float su = fmaxf((float)ds(u, (unsigned)far < (unsigned)n ? far : u), 1.f);
-  const double2 pu = coords[u];
   for (int s0 = 0; s0 < PK; s0 += 32) {
     const int s = s0 + lane;
     const int v = s < PK ? __ldg(mine + s) : -1;
@@ -372,31 +398,31 @@ __global__ void __launch_bounds__(256) edge_features_kernel(const double2* __res
       for (int b = 0; b < B; ++b)
         if (lane == t0 + b) rvu = at[b];
     }
-    if (s >= PK) continue;
-    float f[MLP_F] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    float label = 0.f;
-    if ((unsigned)v < (unsigned)n) {
-      const double2 pv = coords[v];
-      f[0] = (float)ds(u, v) / su;
-      f[1] = (float)s / (float)PK;
-      f[2] = (float)rvu / (float)PK;
-      f[3] = (float)(pv.x - pu.x) / su;
-      f[4] = (float)(pv.y - pu.y) / su;
-      if (tour_pos) {
-        const int pu_ = tour_pos[u], pv_ = tour_pos[v];
-        const int dpos = pu_ > pv_ ? pu_ - pv_ : pv_ - pu_;
-        label = (dpos == 1 || dpos == n - 1) ? 1.f : 0.f;
-      }
-    }
-    const long long e = (long long)u * PK + s;
-    uint32_t* row = X32 + e * 8;
-    row[0] = pack_bf16(f[0], f[1]);
-    row[1] = pack_bf16(f[2], f[3]);
-    row[2] = pack_bf16(f[4], 0.f);
-#pragma unroll
-    for (int q = 3; q < 8; ++q) row[q] = 0u;
-    if (y) y[e] = label;
+    if (s < PK) edge_row(coords, n, ds, tour_pos, u, s, v, PK, su, rvu, X32, y);
   }
+}
+
+// The same with a thread per edge, which walks the neighbour's pool alone.
+__global__ void __launch_bounds__(256) edge_features_thread_kernel(const double2* __restrict__ coords, int n,
+                                                                   const int32_t* __restrict__ pool, int PK, DistSrc ds,
+                                                                   const int32_t* __restrict__ tour_pos,
+                                                                   uint32_t* __restrict__ X32, float* __restrict__ y) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (long long)n * PK) return;
+  const int u = (int)(e / PK), s = (int)(e - (long long)u * PK);
+  const int v = __ldg(pool + e);
+  float su = 1.f;
+  int rvu = PK;
+  if ((unsigned)v < (unsigned)n) {
+    const int far = __ldg(pool + (long long)u * PK + PK - 1);
+    su = fmaxf((float)ds(u, (unsigned)far < (unsigned)n ? far : u), 1.f);
+    for (int q = 0; q < PK; ++q)
+      if (__ldg(pool + (long long)v * PK + q) == u) {
+        rvu = q;
+        break;
+      }
+  }
+  edge_row(coords, n, ds, tour_pos, u, s, v, PK, su, rvu, X32, y);
 }
 
 // Top-k of each node's pool by descending score (ties: lower pool slot first; a NaN is taken
@@ -471,8 +497,16 @@ extern "C" int tspb_edge_features(const double* coords, int32_t n, const int32_t
   ds.dist = dist;
   ds.stride = dist_stride;
   ds.coords = reinterpret_cast<const double2*>(coords);
-  edge_features_kernel<<<(int)(((long long)n + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const double2*>(coords), n, pool, pool_k, ds, tour_pos, reinterpret_cast<uint32_t*>(x), labels);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const double2* xy = reinterpret_cast<const double2*>(coords);
+  uint32_t* rows = reinterpret_cast<uint32_t*>(x);
+  // Short pools leave most lanes of a node's warp idle, and long ones of few nodes leave most SMs
+  // without a warp. n = 50,000, PK = 8 31 us (43 with warps), PK = 16 70 (52); n = 200, PK = 128 24 (36).
+  if (pool_k <= 10 || (pool_k > 32 && (long long)n * pool_k <= 32768))
+    edge_features_thread_kernel<<<(int)(((long long)n * pool_k + 255) / 256), 256, 0, st>>>(xy, n, pool, pool_k, ds,
+                                                                                            tour_pos, rows, labels);
+  else
+    edge_features_kernel<<<(int)(((long long)n + 7) / 8), 256, 0, st>>>(xy, n, pool, pool_k, ds, tour_pos, rows, labels);
   return tspb_launch_status();
 }
 
