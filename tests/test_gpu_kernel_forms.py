@@ -41,6 +41,22 @@ def test_inversion(routes, n):
   assert np.array_equal(d[0].cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("n,pool_k,k", [(30, 12, 7), (30, 13, 13), (32767, 40, 5), (32768, 40, 5), (32768, 31, 31),
+                                        (32768, 32, 3), (32769, 63, 2), (32768, 65, 2)])
+def test_select_topk(n, pool_k, k):
+  torch, native, ptr, stream_handle = _gpu()
+  rng = np.random.default_rng(n + pool_k)
+  pool = rng.integers(0, n, (n, pool_k)).astype(np.int32)
+  score = rng.normal(0.0, 1.0, (n, pool_k)).astype(np.float32)
+  score[1::4] = np.round(score[1::4])  # ties, and zeros of both signs
+  score[2::4] *= rng.choice([1.0, np.inf], (len(score[2::4]), pool_k)).astype(np.float32)
+  out = torch.empty((n, k), dtype=torch.int32, device="cuda")
+  p, s = torch.from_numpy(pool).cuda(), torch.from_numpy(score).cuda()
+  native.call("tspb_select_topk", ptr(p), ptr(s), n, pool_k, k, ptr(out), stream_handle())
+  order = np.argsort(-score, axis=1, kind="stable")[:, :k]
+  assert np.array_equal(out.cpu().numpy(), np.take_along_axis(pool, order, axis=1))
+
+
 @pytest.mark.parametrize("n,pool_k", [(60, 10), (60, 11), (256, 128), (257, 128), (993, 33)])
 @pytest.mark.parametrize("matrix", [True, False])
 def test_edge_features(n, pool_k, matrix):

@@ -482,6 +482,31 @@ __global__ void __launch_bounds__(256) select_topk_kernel(const int32_t* __restr
   }
 }
 
+// The same by a thread per node, which rereads its scores k times.
+__global__ void __launch_bounds__(128) select_topk_thread_kernel(const int32_t* __restrict__ pool,
+                                                                 const float* __restrict__ score, int n, int PK, int k,
+                                                                 int32_t* __restrict__ out) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= n) return;
+  const int32_t* p = pool + (long long)u * PK;
+  const float* sc = score + (long long)u * PK;
+  unsigned long long taken[2] = {0ull, 0ull};  // PK <= 128
+  for (int r = 0; r < k; ++r) {
+    int best = -1;
+    float bs = 0.f;
+    for (int q = 0; q < PK; ++q) {
+      if (taken[q >> 6] & (1ull << (q & 63))) continue;
+      const float s = __ldg(sc + q);
+      if (best < 0 || s > bs) {
+        best = q;
+        bs = s;
+      }
+    }
+    taken[best >> 6] |= 1ull << (best & 63);
+    out[(long long)u * k + r] = __ldg(p + best);
+  }
+}
+
 }  // namespace tspb
 
 using namespace tspb;
@@ -554,7 +579,14 @@ extern "C" int tspb_select_topk(const int32_t* pool, const float* scores, int32_
   if (!pool || !scores || !out) return TSPB_ERR_ARG;
   const int blocks = (int)(((long long)n + 7) / 8);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (pool_k <= 32) select_topk_kernel<1><<<blocks, 256, 0, st>>>(pool, scores, n, pool_k, k, out);
+  // A thread per node where the pool is short, or where nodes are so many that a warp each costs
+  // more than the scattered reads do (pool sizes divisible by 32 excepted: the rows then lie 128 bytes apart,
+  // and the thread form is two to four times slower). n = 50,000: PK = 8, k = 5 11 us (21 with warps), PK = 16, k = 16 31 (40), PK = 40, k = 36 111
+  // (153), PK = 32, k = 10 67 (29); n = 20,000: PK = 16, k = 8 16 either way, PK = 64, k = 20 164 (44).
+  if (pool_k <= 12 || (n >= 32768 && pool_k < 64 && pool_k % 32 != 0))
+    select_topk_thread_kernel<<<(n + 127) / 128, 128, 0, st>>>(pool, scores, n, pool_k, k, out);
+  else if (pool_k > 32 && pool_k <= 64) select_topk_kernel<2><<<blocks, 256, 0, st>>>(pool, scores, n, pool_k, k, out);
+  else if (pool_k <= 32) select_topk_kernel<1><<<blocks, 256, 0, st>>>(pool, scores, n, pool_k, k, out);
   else select_topk_kernel<4><<<blocks, 256, 0, st>>>(pool, scores, n, pool_k, k, out);
   return tspb_launch_status();
 }
