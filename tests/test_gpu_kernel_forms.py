@@ -88,3 +88,19 @@ def test_edge_features(n, pool_k, matrix):
               stream_handle())
   assert torch.equal(got.cpu(), want)
   assert np.array_equal(lab.cpu().numpy(), y)
+
+
+@pytest.mark.parametrize("edges", [6 * 148 * 64 * 16 - 15, 6 * 148 * 64 * 16 + 1])
+def test_mlp_infer_grids(edges):
+  """A row's logit does not depend on the grid: the same rows in a call of their own."""
+  torch, native, ptr, stream_handle = _gpu()
+  gen = torch.Generator().manual_seed(edges)
+  params = (torch.randn(native.load_library().tspb_mlp_param_count(), generator=gen) * 0.1).cuda()
+  x = torch.randn((edges, 16), generator=gen).to(torch.bfloat16).view(torch.int16).cuda()
+  got = torch.empty(edges, device="cuda")
+  native.call("tspb_mlp_infer", ptr(params), ptr(x), edges, ptr(got), stream_handle())
+  for lo in (0, 16 * 1000, edges - 1 - (edges - 1) % 16):
+    rows = min(160, edges - lo)
+    part = torch.empty(rows, device="cuda")
+    native.call("tspb_mlp_infer", ptr(params), ptr(x[lo:lo + rows].contiguous()), rows, ptr(part), stream_handle())
+    assert torch.equal(got[lo:lo + rows], part)
