@@ -23,6 +23,7 @@
 // four entries of a row per thread and skip the distance gather of entries whose lower bound
 // d(a,c) - d(a,b) - d(c,d) is not negative (distances are >= 0).
 #include <algorithm>
+#include <type_traits>
 
 #include "two_opt.cuh"
 
@@ -64,10 +65,10 @@ struct PairList {
   }
 };
 
-// Appends the improving pairs of a warp, up to U per lane (gain < 0, scan index e0 + u, row i,
-// position j[u]), with one shared atomic, and lowers the lane's smallest.
+// Appends the improving pairs of a warp, up to U per lane (gain < 0, scan index e, window
+// i << 16 | j), with one shared atomic, and lowers the lane's smallest.
 template <int U>
-__device__ __forceinline__ void append_pairs(const int (&gain)[U], unsigned e0, int i, const int (&j)[U],
+__device__ __forceinline__ void append_pairs(const int (&gain)[U], const unsigned (&e)[U], const unsigned (&win)[U],
                                              unsigned* count, const PairList& list, Pair& best) {
   unsigned m[U], total = 0;
 #pragma unroll
@@ -83,11 +84,24 @@ __device__ __forceinline__ void append_pairs(const int (&gain)[U], unsigned e0, 
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (gain[u] < 0) {
-      const Pair v{gain_key(gain[u], e0 + u), ((unsigned)i << 16) | (unsigned)j[u]};
+      const Pair v{gain_key(gain[u], e[u]), win[u]};
       if (v.key < best.key) best = v;
       list.put(base + __popc(m[u] & ((1u << lane) - 1u)), v);
     }
     base += __popc(m[u]);
+  }
+}
+
+// d(a[u], b[u]) for the entries with ok[u] (0 elsewhere), all loads in flight together.
+template <int U>
+__device__ __forceinline__ void gather_pairs(const DistSrc& ds, const int (&a)[U], const int (&b)[U],
+                                             const bool (&ok)[U], int (&d)[U]) {
+  if (ds.dist != nullptr) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u] = load_cg_if(ok[u], ds.dist + (long long)a[u] * ds.stride + b[u]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) d[u] = ok[u] ? ds(a[u], b[u]) : 0;
   }
 }
 
@@ -188,11 +202,10 @@ __global__ void __launch_bounds__(1024) two_opt_multi_kernel(const TwoOptArgs A)
       const int di = T / G, dg = T - di * G;
       for (int it0 = wid * 32; it0 < items; it0 += T) {
         const int it = it0 + lane;
-        int gain[4] = {0, 0, 0, 0}, j[4] = {0, 0, 0, 0};
-        unsigned e0 = 0;
+        int gain[4] = {0, 0, 0, 0}, j[4];
+        unsigned e[4] = {}, win[4] = {};
         if (it < items) {
           const unsigned r0 = (unsigned)g * 4u;
-          e0 = (unsigned)i * (unsigned)k + r0;
           const int a = s_tour[i], b = s_tour[i + 1], ea = s_edge[i];
           const uint4 w4 = __ldg(reinterpret_cast<const uint4*>(packed + ((unsigned)a * (unsigned)k + r0)));
           const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
@@ -212,9 +225,13 @@ __global__ void __launch_bounds__(1024) two_opt_multi_kernel(const TwoOptArgs A)
           }
           gather_if(ds, b, d, ok, dbd);
 #pragma unroll
-          for (int u = 0; u < 4; ++u) gain[u] = ok[u] ? lb[u] + dbd[u] : 0;
+          for (int u = 0; u < 4; ++u) {
+            gain[u] = ok[u] ? lb[u] + dbd[u] : 0;
+            e[u] = (unsigned)i * (unsigned)k + r0 + (unsigned)u;
+            win[u] = ((unsigned)i << 16) | (unsigned)j[u];
+          }
         }
-        append_pairs(gain, e0, i, j, &S.m, list, best);
+        append_pairs(gain, e, win, &S.m, list, best);
         i += di;
         g += dg;
         if (g >= G) {
@@ -223,37 +240,62 @@ __global__ void __launch_bounds__(1024) two_opt_multi_kernel(const TwoOptArgs A)
         }
       }
     } else if constexpr (SCAN == MULTI_CAND) {
+      constexpr int U = 4;  // entries of a lane with their loads in flight together
       const int E = rows * k;
-      for (int e0 = wid * 32; e0 < E; e0 += T) {
-        const int e = e0 + lane, i = e / k;
-        int gain[1] = {0}, j[1] = {0};
-        if (e < E) {
-          const int a = s_tour[i];
-          const long long at = (long long)a * k + (e - i * k);
-          const int c = __ldg(cand + at);
-          j[0] = (unsigned)c < (unsigned)n ? s_pos[c] : 0;
-          if (j[0] > i + 1 && j[0] < n - (i == 0)) {
-            ++my_pairs;
-            const int dac = A.cand_dist ? __ldg(A.cand_dist + at) : ds(a, c);
-            gain[0] = (dac - s_edge[i]) + (ds(s_tour[i + 1], s_tour[j[0] + 1 == n ? 0 : j[0] + 1]) - s_edge[j[0]]);
-          }
+      for (int e0 = wid * 32 * U; e0 < E; e0 += T * U) {
+        int gain[U], b[U], d[U], cut[U], dac[U], dbd[U];
+        unsigned e[U], win[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int at = e0 + 32 * u + lane;
+          ok[u] = at < E;
+          const int i = ok[u] ? at / k : 0, a = s_tour[i];
+          const long long f = (long long)a * k + (ok[u] ? at - i * k : 0);
+          const int c = (int)load_nc_if(ok[u], cand + f);
+          const int j = (unsigned)c < (unsigned)n ? s_pos[c] : 0;
+          ok[u] = ok[u] && j > i + 1 && j < n - (i == 0);
+          my_pairs += ok[u];
+          dac[u] = A.cand_dist ? (int)load_nc_if(ok[u], A.cand_dist + f) : (ok[u] ? ds(a, c) : 0);
+          b[u] = s_tour[i + 1];
+          d[u] = s_tour[j + 1 == n ? 0 : j + 1];
+          cut[u] = s_edge[i] + s_edge[j];
+          e[u] = (unsigned)at;
+          win[u] = ((unsigned)i << 16) | (unsigned)j;
         }
-        append_pairs(gain, (unsigned)e, i, j, &S.m, list, best);
+        gather_pairs(ds, b, d, ok, dbd);
+#pragma unroll
+        for (int u = 0; u < U; ++u) gain[u] = ok[u] ? dac[u] - cut[u] + dbd[u] : 0;
+        append_pairs(gain, e, win, &S.m, list, best);
       }
     } else {
       for (int i = wid; i < rows; i += nwarps) {
         const int a = s_tour[i], b = s_tour[i + 1], eab = s_edge[i];
         const int lim = n - (i == 0);
-        for (int j0 = i + 2; j0 < lim; j0 += 32) {
-          const int j[1] = {j0 + lane};
-          int gain[1] = {0};
-          if (j[0] < lim) {
-            ++my_pairs;
-            const int c = s_tour[j[0]], d = s_tour[j[0] + 1 == n ? 0 : j[0] + 1];
-            gain[0] = (ds(a, c) - eab) + (ds(b, d) - s_edge[j[0]]);
+        auto pairs = [&](auto wide, int j0) {  // of U x 32 positions from j0 on
+          constexpr int U = decltype(wide)::value;
+          int gain[U], c[U], d[U], dac[U], dbd[U];
+          unsigned e[U], win[U];
+          bool ok[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int j = j0 + 32 * u + lane;
+            ok[u] = j < lim;
+            my_pairs += ok[u];
+            c[u] = s_tour[ok[u] ? j : 0];
+            d[u] = s_tour[ok[u] && j + 1 < n ? j + 1 : 0];
+            e[u] = (unsigned)i * (unsigned)n + (unsigned)j;
+            win[u] = ((unsigned)i << 16) | (unsigned)j;
           }
-          append_pairs(gain, (unsigned)i * (unsigned)n + (unsigned)j[0], i, j, &S.m, list, best);
-        }
+          gather_if(ds, a, c, ok, dac);
+          gather_if(ds, b, d, ok, dbd);
+#pragma unroll
+          for (int u = 0; u < U; ++u) gain[u] = ok[u] ? (dac[u] - eab) + (dbd[u] - s_edge[win[u] & 0xffffu]) : 0;
+          append_pairs(gain, e, win, &S.m, list, best);
+        };
+        int j0 = i + 2;
+        for (; lim - j0 > 64; j0 += 128) pairs(std::integral_constant<int, 4>{}, j0);
+        for (; j0 < lim; j0 += 32) pairs(std::integral_constant<int, 1>{}, j0);
       }
     }
 
@@ -343,14 +385,18 @@ int launch_two_opt_multi(const TwoOptArgs& args, int threads, size_t smem, cudaS
               : scan == MULTI_CAND ? (a.arrays_in_smem ? two_opt_multi_kernel<MULTI_CAND, true> : two_opt_multi_kernel<MULTI_CAND, false>)
                                    : (a.arrays_in_smem ? two_opt_multi_kernel<MULTI_ALL, true> : two_opt_multi_kernel<MULTI_ALL, false>);
   // Pairs in shared memory, as many as a CTA's share of the SM leaves when as many CTAs run on
-  // it as the batch and the CTA size allow; a pass has at most about half of all entries.
+  // it as the batch and the CTA size allow; a pass has at most about half of all entries. The
+  // plain scans leave the L1 a third of the SM: their loads in flight need room there. Ten passes
+  // from tours along strips: 600 tours of 1000 cities, k = 7 0.64 ms (1.16 with the whole SM for
+  // pairs and one entry a lane in flight); every pair of 16 tours of 2000 cities, five passes 8.5 (13.4).
   const int sms = device_attr(cudaDevAttrMultiProcessorCount);
   const int sm_bytes = device_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
   if (sms > 0 && sm_bytes > 0) {
     int resident = (a.num_tours + sms - 1) / sms;
     resident = std::max(1, std::min(resident, 2048 / threads));
     const long long arrays = (long long)((smem + 15) / 16 * 16);
-    const long long share = std::min<long long>(sm_bytes / resident - 1024, smem_optin()) - (long long)sizeof(MultiSmem) - arrays;
+    const long long usable = scan == MULTI_PACKED ? sm_bytes : sm_bytes / 3 * 2;
+    const long long share = std::min<long long>(usable / resident - 1024, smem_optin()) - (long long)sizeof(MultiSmem) - arrays;
     const long long rows = a.n - 2;
     const long long most = scan == MULTI_ALL ? rows * (rows + 1) / 2 : rows * a.k;
     const long long cap = std::min(share / 12, most) & ~1LL;
