@@ -1,4 +1,4 @@
-// GRASP nearest-neighbour initial tours, one thread per row, bit-identical to the
+// GRASP nearest-neighbour initial tours, one thread or one warp per row, bit-identical to the
 // reference's `_nearest_neighbor_row_cpu`
 // (src/algorithms/strategies/initialization/nearest_neighbor_init.py:31-99) with the
 // SplitMix64 stream of src/utils/splitmix64.py:38-51:

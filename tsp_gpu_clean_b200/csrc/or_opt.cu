@@ -24,8 +24,8 @@
 //     k-NN table for entries whose candidate has a new successor: such an entry is evaluated
 //     alone, unless it was its row's minimum, which makes the row one of the first kind.
 // The table is scanned rather than indexed by candidate: four words a load, four
-// to six instructions a word, the same for any table, against a reverse index that every call
-// would build first.
+// to six instructions a word, the same for any table. The entry point takes no reverse index;
+// for a table that has one, its lists of the changed cities would be the shorter way.
 //
 // Measured: 1024 tours of 1000 cities, k = 20, segments up to 3, 50 passes 2.34 ms (27.2 with
 // a whole scan each pass); the first scan is 0.47 ms of it, bound by the gathers (32 bytes of

@@ -10,7 +10,8 @@
 //   - a move is up to three reversals: [i+1, j] (cases 1, 4, 5, 7), [j+1, k] (2, 4, 5, 6),
 //     [i+1, k] (3, 5, 6, 7).
 //
-// What bounds it: integer issue. A pass is n^3/6 triples and everything it reads is the
+// What bounds it: instruction issue, and the latency between (issue slots 61 % busy on the SMs
+// that hold a CTA; ncu, 32 tours of 200 cities). A pass is n^3/6 triples and everything it reads is the
 // tour-ordered matrix M[p][q] = d(t[p], t[q]), so the layout is chosen to spend as few
 // instructions per triple as possible.
 //   - Cases 1, 2 and 3 are the same 2-opt moves met again and again: the pair (x, y) is case 2
@@ -20,8 +21,10 @@
 //     (one per lane) and walks j: the rows i .. i+4 at columns k and k+1 stay in registers,
 //     two coalesced reads (M[j][k], M[j+1][k+1]) serve all four i, and the terms that depend
 //     on (i, j) alone are computed once per unit by 16 lanes and read back as three 16-byte
-//     broadcasts per j. About 12 instructions per 32 triples; the former layout (a warp per
-//     (i, j), int64, all six cases per triple) took about 180.
+//     broadcasts per j. About 12 instructions per 32 triples where no lane has a move at or below
+//     its best, 34 on average over ten passes from random tours (the units' set-up, and lanes with
+//     such a move send their warp through the keys); the former layout (a warp per (i, j), int64,
+//     all six cases per triple) took about 180.
 //   - Deltas are int32 when every distance of M is below 2^29 (three of them fit), int64
 //     otherwise; the choice is made per tour from M itself.
 //   - A batch with fewer tours than SMs gives each tour a cluster of 2, 4 or 8 CTAs, the

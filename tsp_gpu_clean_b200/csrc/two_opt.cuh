@@ -33,9 +33,6 @@ struct TwoOptArgs {
 __device__ __forceinline__ unsigned long long gain_key(int gain, unsigned idx) {
   return ((unsigned long long)((unsigned)gain ^ 0x80000000u) << 32) | idx;
 }
-__device__ __forceinline__ int key_gain(unsigned long long key) {
-  return (int)((unsigned)(key >> 32) ^ 0x80000000u);
-}
 
 constexpr unsigned long long NO_KEY = ~0ull;
 constexpr unsigned NO_IDX = ~0u;

@@ -30,7 +30,7 @@
 // What bounds it: the chain of a unit (city, row lookups, shuffles, two warp reductions a row)
 // and, for tiles, their copies from L2. Measured through the strategy, before and after: 128
 // tours of 500 cities to a local optimum, best 59.5 -> 10.8 ms, first 124.1 -> 20.8 ms; 100 of
-// 100 cities, best 0.89 -> 0.53 ms; one of 200 cities, ten passes 0.31 -> 0.20 ms.
+// 100 cities, best 0.89 -> 0.53 ms; one of 200 cities, ten passes 0.29 -> 0.18 ms.
 #include <algorithm>
 
 #include "two_opt.cuh"
