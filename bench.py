@@ -67,8 +67,8 @@ L2_FLUSH_BYTES = 256 << 20
 #: DRAM bytes read + written scaled to a 1024-tour launch (the tours' 4 KB each is the part
 #: that grows). A gain is computed only for entries whose lower bound could improve.
 NCU_PER_GAIN: dict[str, dict[str, float]] = {
-  "first": {"inst": 8.337, "lts_bytes": 32.52, "dram_bytes_per_launch": 8_486_144},
-  "best": {"inst": 9.083, "lts_bytes": 31.95, "dram_bytes_per_launch": 8_617_472},
+  "first": {"inst": 7.331, "lts_bytes": 32.10, "dram_bytes_per_launch": 8_423_168},
+  "best": {"inst": 20.336, "lts_bytes": 36.62, "dram_bytes_per_launch": 8_492_800},
 }
 #: CPU parity sample: tours of the timed batch refined by the oracle (at least this many)
 PARITY_TOURS = 16
